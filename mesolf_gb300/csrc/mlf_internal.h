@@ -181,7 +181,7 @@ struct Solver {
   DevBuf Xtmp;       // float [nch][plane]      scratch volume (back-projection output, filter)
   DevBuf lfs;        // float [N*N][Lj*Li]      sub-aperture images
   DevBuf rpad;       // float [RProws][RP]      halo-padded ratio image
-  DevBuf part;       // float [grid*slots][tilesB*VW_TY][tilesA*VW_TX] per-slot forward partials
+  DevBuf part;       // float [grid][slots][tilesB*VW_TY][tilesA*VW_TX] per-slot forward partials
   DevBuf hx;         // float [Lj*Li]           last forward projection
   DevBuf cls;        // int tables: clsA[3][Li], clsB[3][Lj], rngA[3][maxc][2], rngB[3][maxc][2]
   DevBuf red;        // double scratch for reductions
@@ -341,6 +341,8 @@ constexpr int VW_TY = 4;
 constexpr int VW_TX = 8;
 // threads per view-kernel CTA at most (two slots of up to 160 tiles)
 constexpr int kViewMaxThreads = 320;
+// Whether a CTA adds its slots' forward partials itself (the comment at the sum in k_view).
+__host__ __device__ constexpr bool view_sums_slots(int slots) { return slots > 2; }
 // Staged planes of the view kernel (ratio image, forward input) are stored with their
 // 16-byte column chunks swizzled: in every other 32-float block the chunks of each pair
 // trade places (column c lives at c ^ 4 when bit 5 of c is set), except a last chunk whose

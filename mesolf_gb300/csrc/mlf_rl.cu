@@ -206,10 +206,11 @@ __global__ void k_scatter_views(const float* __restrict__ lfs, PatchGeo g, float
 // ratio image R = LF_sub ./ HX with non-finite -> 0 (recon_…_with_filter.m:116-117) into
 // the halo-padded buffer read by the next view kernel.  A partial plane holds row b of the
 // lenslet grid at b * HP (HP >= Li, the view kernel's tile-padded width), planes PPL floats
-// apart.  One block covers 32 positions (lanes); its 8 warps take the partials k = w, w+8,
-// ... with four accumulators each, and the warps' sums are added in a fixed order
-// (deterministic).
-constexpr int kReduceGroups = 8;
+// apart.  One block covers 32 positions (lanes); its warps take the partials k = w, w +
+// kReduceGroups, ... and their sums are added in a fixed order (deterministic).  Bound by the
+// latency of the L2 reads, so 32 warps share the planes (31 x 40 lenslets: 22.6 us for 1824
+// slot planes on 8 warps, 4.2 us for the 456 planes that the CTAs leave on 32).
+constexpr int kReduceGroups = 32;
 __global__ void __launch_bounds__(32 * kReduceGroups)
 k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int HP, int64_t PPL,
                const float* __restrict__ lfsub, float* __restrict__ hx_out,
@@ -224,6 +225,7 @@ k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int H
   if (i < LL) {
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
     int k = grp;
+#pragma unroll 3
     for (; k + 3 * kReduceGroups < nparts; k += 4 * kReduceGroups) {
       s0 += pp[k * PPL];
       s1 += pp[(k + kReduceGroups) * PPL];
@@ -365,8 +367,9 @@ int run_reduce(Solver* s, int view, float* hx_out, bool ratio, cudaStream_t st) 
   const int LL = s->Li * s->Lj;
   const float* lfsub = s->lfs.as<float>() + (int64_t)view * LL;
   const int HP = s->tilesA * VW_TX;
+  const int group = view_sums_slots(s->slots) ? s->slots : 1;  // planes that the view kernel has added
   k_reduce_ratio<<<ceil_div(LL, 32), 32 * kReduceGroups, 0, st>>>(
-      s->part.as<float>(), s->grid * s->slots, s->Li, s->Lj, HP, (int64_t)s->tilesB * VW_TY * HP, lfsub, hx_out,
+      s->part.as<float>(), s->grid * s->slots / group, s->Li, s->Lj, HP, (int64_t)group * s->tilesB * VW_TY * HP, lfsub, hx_out,
       ratio ? s->rpad.as<float>() : nullptr, s->RP, s->q + 1);
   MLF_LAUNCHED();
   return MLF_OK;
