@@ -16,9 +16,15 @@
 // of one column (coalesced along the fast axis of the output, which maps to
 // near-consecutive raw rows) and 8 output frames, with all 32 neighbour loads of the 8
 // frames in flight before the interpolation.  One input frame per output frame
-// (k_rectify_staged): the raw tile of a block is staged in shared memory by 16-byte copies
-// and the next frame chunk is prefetched while the current one is interpolated.  The raw
-// data is read once from HBM.
+// (k_rectify_rows): the raw tile of a block is staged in shared memory by 16-byte copies
+// and the next frame chunk is prefetched while the current one is interpolated.
+//
+// The division by the movie's maximum needs the maximum first.  One input frame per output
+// frame: the interpolation runs twice, first for the maximum alone (reads the raw cut, writes
+// nothing), then writing the divided values, so the movie is written once and never read back:
+// 2 x 2 + 4 bytes per pixel of 16-bit frames where write, maximum and scaling passes moved 18.
+// Averaged frames read navg frames per output, so there the write pass takes the maximum and a
+// scaling pass follows (2 navg + 12 bytes).
 #include "mlf_internal.h"
 
 #include <algorithm>
@@ -40,17 +46,31 @@ __device__ __forceinline__ float ldv(const TIn* p) {
 // Block: RC_ROWS output rows x RC_COLS columns (threadIdx.y), output frames in chunks of
 // RC_FCH (all 4*RC_FCH neighbour loads of a chunk in flight before the interpolation), RC_NCH
 // chunks per block; the tables are read once per thread.
+// max_part (nullable): the largest value of each block.
 constexpr int RC_ROWS = 128, RC_COLS = 4, RC_FCH = 8, RC_NCH = 8;
+
+// Maximum over the block (fmaxf: NaN only where every value is NaN), valid in thread 0.
+__device__ __forceinline__ float rc_block_max(float m, float* sh) {
+  const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
+  if ((tid & 31) == 0) sh[tid >> 5] = m;
+  __syncthreads();
+  if (tid == 0)
+    for (int w = 1; w < (int)(blockDim.x * blockDim.y >> 5); ++w) m = fmaxf(m, sh[w]);
+  return m;
+}
 
 template <typename TIn>
 __global__ void __launch_bounds__(RC_ROWS * RC_COLS)
 k_rectify(const TIn* __restrict__ raw, int64_t fstride, int64_t cstride, int64_t row0, int64_t col0,
           const int* __restrict__ iy, const float* __restrict__ wy, int oh, const int* __restrict__ ix,
           const float* __restrict__ wx, int ow, int64_t f0, int64_t fstep, int navg, int64_t flast, int64_t n_out,
-          float* __restrict__ out) {
+          float* __restrict__ out, float* __restrict__ max_part) {
+  __shared__ float mx_sh[32];
   const int r = blockIdx.x * RC_ROWS + threadIdx.x;
   const int c = blockIdx.y * RC_COLS + threadIdx.y;
-  if (r >= oh || c >= ow) return;
+  float mx = -INFINITY;
+  if (r < oh && c < ow) {
   const int64_t P = (int64_t)oh * ow;
   const int i0 = __ldg(iy + r), j0 = __ldg(ix + c);
   const float fy = __ldg(wy + r), fx = __ldg(wx + c);
@@ -59,7 +79,7 @@ k_rectify(const TIn* __restrict__ raw, int64_t fstride, int64_t cstride, int64_t
   float* op = out + r + (int64_t)oh * c;
   for (int ch = 0; ch < RC_NCH; ++ch) {
     const int64_t ib = ((int64_t)blockIdx.z * RC_NCH + ch) * RC_FCH;
-    if (ib >= n_out) return;
+    if (ib >= n_out) break;
     const int ni = (int)(n_out - ib < RC_FCH ? n_out - ib : RC_FCH);
     if (navg == 1) {
       float v[RC_FCH][4];
@@ -77,7 +97,9 @@ k_rectify(const TIn* __restrict__ raw, int64_t fstride, int64_t cstride, int64_t
       for (int q = 0; q < RC_FCH; ++q) {
         if (q < ni) {
           const float a = fmaf(fx, v[q][2] - v[q][0], v[q][0]), b = fmaf(fx, v[q][3] - v[q][1], v[q][1]);
-          __stcs(op + P * (ib + q), fmaf(fy, b - a, a));
+          const float o = fmaf(fy, b - a, a);
+          mx = fmaxf(mx, o);
+          __stcs(op + P * (ib + q), o);
         }
       }
       continue;
@@ -95,147 +117,274 @@ k_rectify(const TIn* __restrict__ raw, int64_t fstride, int64_t cstride, int64_t
       }
       const float rn = 1.f / (float)(fb - fa + 1);
       const float a = fmaf(fx, v01 - v00, v00), b = fmaf(fx, v11 - v10, v10);
-      __stcs(op + P * (ib + q), fmaf(fy, b - a, a) * rn);
+      const float o = fmaf(fy, b - a, a) * rn;
+      mx = fmaxf(mx, o);
+      __stcs(op + P * (ib + q), o);
     }
+  }
+  }
+  if (max_part) {
+    const float m = rc_block_max(mx, mx_sh);
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+      max_part[((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = m;
   }
 }
 
-// The same for one input frame per output frame (navg = 1), with the raw tile of each block
-// staged in shared memory by 16-byte loads: block = RC_ROWS x RC_COLS output pixels, chunks of
-// SF output frames (blockIdx.z).  For frame q and raw column k of the block's footprint (raw
-// columns ix[c0] .. ix[c1]+1, rows iy[r0] .. iy[r1]+1) the column segment is loaded from the
-// 16-byte boundary at or below its first element into slot [q][k] (`slot` elements), its
-// start at off[q][k] inside the slot.  A few wide loads per thread replace four narrow
-// gathers per output pixel and frame.  raw must be 16-byte aligned; `total` = elements of
-// the frame buffer (vectors that would cross its end are loaded per element).
-constexpr int SF = 16;
+// One input frame per output frame, with the raw tile of each block staged in shared memory by
+// 16-byte loads.  Block = blockDim.x output rows (32 .. RR_MAX_ROWS) x RR_COLS output columns; stages of
+// RR_SF output frames, two per thread (threadIdx.y picks the pair).  For frame q and raw column
+// k of the block's footprint (raw columns ix[c0] .. ix[c1]+1, rows iy[r0] .. iy[r1]+1) the
+// column segment is loaded from the 16-byte boundary at or below its first element into slot
+// [q][k] (`slot` elements).  raw must be 16-byte aligned; `total` = elements of the frame buffer
+// (bytes past its end are zero-filled, never read).
+//
+// Bound: instruction issue (82 % of the slots with one thread per output pixel, which took all
+// four neighbours per output: 20 instructions), then HBM.  So a thread walks RR_COLS output
+// columns of its row: the interpolation along the row axis is done once per raw column and
+// serves the outputs on both sides of it, and its two frames share addresses, tables and packed
+// FP32 instructions.  2000 frames of 1100 x 1100 16-bit pixels to 1065 x 1065: maximum pass
+// 1.92 ms (issue 84 %), writing pass 2.95 ms (4.6 TB/s); before, interpolation 3.35, maximum 1.51
+// and scaling 5.03 ms.
+constexpr int RR_COLS = 16, RR_SF = 4, RR_MAX_ROWS = 160;
+enum RectifyMode { RR_PLAIN = 0, RR_MAX = 1, RR_DIV = 2 };
 
-// exact uint16 -> float with one logic op and one add: the bits 0x4B000000 | x are the float
-// 2^23 + x (x < 2^23 fits the mantissa)
-__device__ __forceinline__ float to_f(uint16_t x) { return __uint_as_float(0x4B000000u | x) - 8388608.f; }
-__device__ __forceinline__ float to_f(float x) { return x; }
+// exact uint16 -> float: the bits 0x4B000000 | x are the float 2^23 + x (x < 2^23 fits the
+// mantissa), and 2^23 is taken out where the value itself is needed
+__device__ __forceinline__ float rr_raw(uint16_t x) { return __uint_as_float(0x4B000000u | x); }
+__device__ __forceinline__ float rr_raw(float x) { return x; }
+
+using f32x2 = unsigned long long;  // two FP32 values (lower half: the thread's first frame)
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 
 __device__ __forceinline__ void rc_cp_async16(void* smem, const void* gmem, int src_bytes) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(src_bytes) : "memory");
 }
 
-// Persistent over frame chunks z = blockIdx.z, blockIdx.z + gridDim.z, ...: the raw tile of
-// chunk z+1 is copied into the second buffer (16-byte zero-filling cp.async, no register
-// round trip) while chunk z is interpolated, so DRAM loads stay in flight.
-template <typename TIn>
-__global__ void __launch_bounds__(RC_ROWS * RC_COLS, 3)
-k_rectify_staged(const TIn* __restrict__ raw, int64_t total, int64_t fstride, int64_t cstride, int64_t row0,
-                 int64_t col0, const int* __restrict__ iy, const float* __restrict__ wy, int oh,
-                 const int* __restrict__ ix, const float* __restrict__ wx, int ow, int64_t f0, int64_t fstep,
-                 int64_t n_out, int slot, int maxc, int same_align, float* __restrict__ out) {
+struct RectifyRows {
+  int64_t total, fstride, cstride, row0, col0;
+  const int* iy;
+  const float* wy;
+  const int* ix;
+  const float* wx;
+  int oh, ow;
+  int64_t f0, fstep, n_out;
+  int slot, maxc;
+  const float* mx;   // RR_DIV: the movie's maximum
+  float* max_part;   // RR_MAX: largest value per block
+};
+
+// Persistent over stages z = blockIdx.z, blockIdx.z + gridDim.z, ...: the raw tile of stage z+1
+// is copied into the second buffer (16-byte zero-filling cp.async, no register round trip)
+// while stage z is interpolated, so DRAM loads stay in flight.  SAME: every frame starts at the
+// same offset from a 16-byte boundary, so a column's place in its slot is one table entry.
+template <typename TIn, int MODE, bool SAME>
+__global__ void __launch_bounds__(2 * RR_MAX_ROWS)
+k_rectify_rows(const TIn* __restrict__ raw, RectifyRows A, float* __restrict__ out) {
   constexpr int VEC = 16 / sizeof(TIn);
-  constexpr int NT = RC_ROWS * RC_COLS;
   extern __shared__ __align__(16) unsigned char rc_smem[];
-  TIn* tiles = reinterpret_cast<TIn*>(rc_smem);  // [2 buffers][SF][maxc][slot]
-  __shared__ int off[2][SF][8];
-  const int tid = threadIdx.y * RC_ROWS + threadIdx.x;
-  const int r0 = blockIdx.x * RC_ROWS, c0 = blockIdx.y * RC_COLS;
-  const int r1 = min(r0 + RC_ROWS, oh) - 1, c1 = min(c0 + RC_COLS, ow) - 1;
-  const int rlo = __ldg(iy + r0), nrow = __ldg(iy + r1) + 2 - rlo;
-  const int clo = __ldg(ix + c0), ncol = __ldg(ix + c1) + 2 - clo;  // <= maxc (host bound)
-  const int nv = (nrow + 2 * VEC - 2) / VEC;                         // vectors per column segment
-  const int64_t chunks = (n_out + SF - 1) / SF;
-  const int64_t fs = (int64_t)SF * maxc * slot;                    // elements per buffer
-  // staging role of this thread: one (column k, vector v) of the footprint, frames q = g, g+G, ...
+  TIn* tiles = reinterpret_cast<TIn*>(rc_smem);  // [2 buffers][RR_SF][maxc][slot]
+  __shared__ int2 colt[RR_COLS];                 // per output: left raw column, weight; bit 31 of the
+                                                 // column: it is not the previous output's right one
+  __shared__ float mx_sh[32];
+  const int rows = blockDim.x, nthr = 2 * rows;
+  const int tid = threadIdx.y * rows + threadIdx.x;
+  const int r0 = blockIdx.x * rows, c0 = blockIdx.y * RR_COLS;
+  const int r1 = min(r0 + rows, A.oh) - 1, cn = min(RR_COLS, A.ow - c0);
+  const int rlo = __ldg(A.iy + r0), nrow = __ldg(A.iy + r1) + 2 - rlo;
+  const int clo = __ldg(A.ix + c0), ncol = __ldg(A.ix + c0 + cn - 1) + 2 - clo;  // <= maxc (host bound)
+  const int nv = (nrow + 2 * VEC - 2) / VEC;                                     // vectors per column segment
+  const int64_t stages = (A.n_out + RR_SF - 1) / RR_SF;
+  const int per = A.maxc * A.slot;  // elements per staged frame
+  const int64_t base0 = (A.row0 + rlo) + A.cstride * (A.col0 + clo);
+  if (tid < cn) {
+    const int lc = __ldg(A.ix + c0 + tid) - clo;
+    const int prev = tid > 0 ? __ldg(A.ix + c0 + tid - 1) - clo : -2;
+    colt[tid] = make_int2(lc | (lc == prev + 1 ? 0 : (int)0x80000000), __float_as_int(__ldg(A.wx + c0 + tid)));
+  }
+  // vector e of a stage = (frame q, column k, vector v), e = tid, tid + nthr, ...: the first one
+  // and the step from one to the next are divided once
   const int cnv = ncol * nv;
-  const int G = NT / cnv;  // >= 1: the host bounds nrow and maxc
-  const int sg = tid / cnv, srem = tid - sg * cnv;
-  const int sk = srem / nv, sv = srem - sk * nv;
-  const int64_t colbase = (row0 + rlo) + cstride * (col0 + clo + sk);
+  const int q_0 = tid / cnv, k_0 = (tid - q_0 * cnv) / nv, v_0 = tid - q_0 * cnv - k_0 * nv;
+  const int dq = nthr / cnv, dk = (nthr - dq * cnv) / nv, dv = nthr - dq * cnv - dk * nv;
   auto stage = [&](int64_t z, int b) {
-    if (sg >= G) return;
-    const int64_t ib = z * SF;
-    const int nf = (int)(n_out - ib < SF ? n_out - ib : SF);
-    const int64_t fdelta = (int64_t)G * fstep * fstride;
-    int64_t e = (f0 + (ib + sg) * fstep) * fstride + colbase;
-    for (int q = sg; q < nf; q += G, e += fdelta) {
-      const int64_t ea = e & ~(int64_t)(VEC - 1);
-      if (sv == 0) off[b][q][sk] = (int)(e - ea);
-      TIn* dst = tiles + b * fs + ((int64_t)q * maxc + sk) * slot + (int64_t)sv * VEC;
-      const int64_t src = ea + (int64_t)sv * VEC;
-      const int64_t avail = total - src;  // elements of the frame buffer left from src
+    const int64_t ib = z * RR_SF;
+    const int nf = (int)(A.n_out - ib < RR_SF ? A.n_out - ib : RR_SF);
+    const int64_t e0 = (A.f0 + ib * A.fstep) * A.fstride + base0;
+    TIn* const buf = tiles + (int64_t)b * RR_SF * per;
+    int q = q_0, k = k_0, v = v_0;
+    while (q < nf) {
+      const int64_t e = e0 + q * A.fstep * A.fstride + k * A.cstride;
+      const int64_t src = (e & ~(int64_t)(VEC - 1)) + v * VEC;
+      const int64_t avail = A.total - src;  // elements of the frame buffer left from src
       const int nbytes = avail >= VEC ? 16 : (avail > 0 ? (int)avail * (int)sizeof(TIn) : 0);
-      rc_cp_async16(dst, nbytes > 0 ? (const void*)(raw + src) : (const void*)raw, nbytes);
+      rc_cp_async16(buf + q * per + k * A.slot + v * VEC, nbytes > 0 ? (const void*)(raw + src) : (const void*)raw,
+                    nbytes);
+      v += dv;
+      k += dk;
+      q += dq;
+      if (v >= nv) {
+        v -= nv;
+        ++k;
+      }
+      if (k >= ncol) {
+        k -= ncol;
+        ++q;
+      }
     }
   };
-  const int r = r0 + threadIdx.x, c = c0 + threadIdx.y;
-  const bool mine = r < oh && c < ow;
-  const int lr = mine ? __ldg(iy + r) - rlo : 0, lc = mine ? __ldg(ix + c) - clo : 0;
-  const float fy = mine ? __ldg(wy + r) : 0.f, fx = mine ? __ldg(wx + c) : 0.f;
-  const int64_t P = (int64_t)oh * ow;
-  const int per = maxc * slot;  // elements per staged frame
+  const int r = r0 + threadIdx.x;
+  const bool mine = r < A.oh;
+  const int lr = mine ? __ldg(A.iy + r) - rlo : 0;
+  const float fy = mine ? __ldg(A.wy + r) : 0.f;
+  const f32x2 fy2 = pack2(fy, fy), minus1 = pack2(-1.f, -1.f);
+  const int64_t P = (int64_t)A.oh * A.ow;
+  const int cs = (int)(A.cstride & (VEC - 1));
+  float mx = MODE == RR_DIV ? __ldg(A.mx) : -INFINITY;
+  // Division by the maximum.  16-bit frames: q = v * (1/mx), then the correction of q by its
+  // residual, fma(fma(-q, mx, v), 1/mx, q), which is the correctly rounded quotient for a
+  // correctly rounded reciprocal (P. Markstein, IBM J. Res. Dev. 34, 1990) while nothing
+  // overflows or underflows: the values are interpolated integers, and a maximum outside
+  // [2^-10, 2^20] takes the division, as do 32-bit frames.
+  const bool fast_div = MODE == RR_DIV && sizeof(TIn) == 2 && mx >= 0x1p-10f && mx <= 0x1p20f;
+  const float rm = fast_div ? 1.f / mx : 0.f;
+  const f32x2 rm2 = pack2(rm, rm), nmx2 = pack2(-mx, -mx);
   int b = 0;
-  if (blockIdx.z < chunks) stage(blockIdx.z, 0);
+  if (blockIdx.z < stages) stage(blockIdx.z, 0);
   asm volatile("cp.async.commit_group;\n" ::: "memory");
-  for (int64_t z = blockIdx.z; z < chunks; z += gridDim.z, b ^= 1) {
+  for (int64_t z = blockIdx.z; z < stages; z += gridDim.z, b ^= 1) {
     const int64_t zn = z + gridDim.z;
-    if (zn < chunks) stage(zn, b ^ 1);  // the other buffer was last read before the barrier below
+    if (zn < stages) stage(zn, b ^ 1);  // the other buffer was last read before the barrier below
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;\n" ::: "memory");
-    __syncthreads();  // chunk z staged by every thread
-    if (mine) {
-      const int64_t ib = z * SF;
-      const int nf = (int)(n_out - ib < SF ? n_out - ib : SF);
-      float* op = out + r + (int64_t)oh * c + P * ib;
-      const TIn* base = tiles + b * fs + (int64_t)lc * slot + lr;
-      if (same_align) {
-        // every frame has the same 16-byte alignment: the column offsets of frame 0 serve all
-        const TIn* ca = base + off[b][0][lc];
-        const TIn* cb = base + slot + off[b][0][lc + 1];
-#pragma unroll
-        for (int q = 0; q < SF; ++q) {
-          if (q < nf) {
-            const float v00 = to_f(ca[q * per]), v10 = to_f(ca[q * per + 1]);
-            const float v01 = to_f(cb[q * per]), v11 = to_f(cb[q * per + 1]);
-            const float a = fmaf(fx, v01 - v00, v00), bb = fmaf(fx, v11 - v10, v10);
-            __stcs(op + P * q, fmaf(fy, bb - a, a));
+    __syncthreads();  // stage z copied by every thread
+    const int64_t ib = z * RR_SF;
+    const int qa = 2 * threadIdx.y;
+    const int na = (int)(A.n_out - ib < RR_SF ? A.n_out - ib : RR_SF) - qa;  // frames of this thread
+    if (mine && na > 0) {
+      // the second frame repeats the first when there is none (its outputs are not stored)
+      const int sec = na > 1 ? 1 : 0;
+      const TIn* pa = tiles + ((int64_t)b * RR_SF + qa) * per + lr;
+      const TIn* pb = pa + sec * per;
+      const int64_t ea = (A.f0 + (ib + qa) * A.fstep) * A.fstride + base0;
+      const int la = (int)(ea & (VEC - 1)), lb = (int)((ea + sec * A.fstep * A.fstride) & (VEC - 1));
+      // raw column k interpolated along the rows, both frames
+      auto column = [&](int k) {
+        const int oa = k * A.slot + ((la + k * cs) & (VEC - 1));
+        const int ob = SAME ? oa : k * A.slot + ((lb + k * cs) & (VEC - 1));
+        const f32x2 x0 = pack2(rr_raw(pa[oa]), rr_raw(pb[ob])), x1 = pack2(rr_raw(pa[oa + 1]), rr_raw(pb[ob + 1]));
+        const f32x2 a = sizeof(TIn) == 2 ? add2(x0, pack2(-8388608.f, -8388608.f)) : x0;
+        return fma2(fma2(x0, minus1, x1), fy2, a);
+      };
+      float* op = out + r + (int64_t)A.oh * c0 + P * (ib + qa);
+      f32x2 left = 0, right = 0;
+      // few iterations in flight per thread keep the stores of a block close together in memory:
+      // 3.76 / 3.13 / 2.93 ms for the writing pass unrolled 8 / 4 / 2 times
+#pragma unroll(MODE == RR_MAX ? 4 : 2)
+      for (int c = 0; c < cn; ++c) {
+        const int2 t = colt[c];
+        const int lc = t.x & 0x7fffffff;
+        left = right;
+        if (t.x < 0) left = column(lc);  // block-uniform: a raw column was skipped or repeated
+        right = column(lc + 1);
+        const float fx = __int_as_float(t.y);
+        const f32x2 o2 = fma2(fma2(left, minus1, right), pack2(fx, fx), left);
+        if (MODE == RR_MAX) {
+          const float2 o = unpack2(o2);
+          mx = fmaxf(mx, fmaxf(o.x, o.y));
+        } else {
+          float2 o;
+          if (MODE == RR_DIV && fast_div) {
+            const f32x2 q2 = mul2(o2, rm2);
+            o = unpack2(fma2(fma2(q2, nmx2, o2), rm2, q2));
+          } else {
+            o = unpack2(o2);
+            if (MODE == RR_DIV) {
+              o.x = o.x / mx;
+              o.y = o.y / mx;
+            }
           }
-        }
-      } else {
-#pragma unroll 4
-        for (int q = 0; q < nf; ++q) {
-          const TIn* ca = base + (int64_t)q * per + off[b][q][lc];
-          const TIn* cb = base + (int64_t)q * per + slot + off[b][q][lc + 1];
-          const float v00 = to_f(ca[0]), v10 = to_f(ca[1]), v01 = to_f(cb[0]), v11 = to_f(cb[1]);
-          const float a = fmaf(fx, v01 - v00, v00), bb = fmaf(fx, v11 - v10, v10);
-          __stcs(op + P * q, fmaf(fy, bb - a, a));
+          __stcs(op, o.x);
+          if (sec) __stcs(op + P, o.y);
+          op += A.oh;
         }
       }
     }
     __syncthreads();  // buffer b is read: the next iteration may stage into it
   }
   asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (MODE == RR_MAX) {
+    const float m = rc_block_max(mx, mx_sh);
+    if (tid == 0) A.max_part[((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = m;
+  }
 }
 
-__global__ void k_rc_max(const float* __restrict__ a, int64_t n, float* __restrict__ part) {
+// One block: mx = max(part[0..n))
+__global__ void __launch_bounds__(1024) k_rc_max(const float* __restrict__ part, int64_t n, float* __restrict__ mx) {
   __shared__ float sh[32];
   float m = -INFINITY;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, a[i]);
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, sh[w]);
-    part[blockIdx.x] = m;
+  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, part[i]);
+  m = rc_block_max(m, sh);
+  if (threadIdx.x == 0) *mx = m;
+}
+
+// a /= *mx: 4 elements per thread and step (VEC: n % 4 == 0 and a 16-byte aligned).
+template <bool VEC>
+__global__ void __launch_bounds__(256) k_rc_scale(float* __restrict__ a, int64_t n, const float* __restrict__ mx) {
+  const float m = __ldg(mx);
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  if (VEC) {
+    float4* a4 = reinterpret_cast<float4*>(a);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += step) {
+      float4 v = a4[i];
+      v.x = v.x / m;
+      v.y = v.y / m;
+      v.z = v.z / m;
+      v.w = v.w / m;
+      a4[i] = v;
+    }
+  } else {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) a[i] = a[i] / m;
   }
 }
 
-__global__ void k_rc_scale(float* __restrict__ a, int64_t n, const float* __restrict__ part, int nparts) {
-  __shared__ float mx;
-  if (threadIdx.x == 0) {
-    float m = -INFINITY;
-    for (int i = 0; i < nparts; ++i) m = fmaxf(m, part[i]);
-    mx = m;
-  }
-  __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    a[i] = a[i] / mx;
+template <typename TIn, int MODE>
+int launch_rows(const void* raw, const RectifyRows& A, bool same, dim3 grid, dim3 block, size_t smem, float* out,
+                cudaStream_t st) {
+  auto kf = same ? k_rectify_rows<TIn, MODE, true> : k_rectify_rows<TIn, MODE, false>;
+  MLF_TRY(allow_max_dyn_smem((const void*)kf));
+  kf<<<grid, block, smem, st>>>(static_cast<const TIn*>(raw), A, out);
+  MLF_LAUNCHED();
+  return MLF_OK;
+}
+template <int MODE>
+int launch_rows(int dtype, const void* raw, const RectifyRows& A, bool same, dim3 grid, dim3 block, size_t smem,
+                float* out, cudaStream_t st) {
+  return dtype == MLF_DTYPE_U16 ? launch_rows<uint16_t, MODE>(raw, A, same, grid, block, smem, out, st)
+                                : launch_rows<float, MODE>(raw, A, same, grid, block, smem, out, st);
 }
 
 // MATLAB a:d:b (d != 0): count floor((b-a)/d) + 1 with a relative tolerance of 1e-10
@@ -300,71 +449,99 @@ int rectify_run(const void* d_raw, int dtype, int64_t total, int64_t fstride, in
   MLF_CUDA(cudaMemcpyAsync(d_wy, wy.data(), sizeof(float) * out_h, cudaMemcpyHostToDevice, st));
   MLF_CUDA(cudaMemcpyAsync(d_wx, wx.data(), sizeof(float) * out_w, cudaMemcpyHostToDevice, st));
   const int64_t P = out_h * out_w;
+  int dev = 0, nsm = 0;
+  MLF_CUDA(cudaGetDevice(&dev));
+  MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // rows per block: of 96, 128 and 160 (the whole image's warps below 96) the one that covers
+  // out_h with the fewest idle lanes, the larger on a tie.  Shorter runs of rows write partial
+  // sectors at both ends too often (1065 rows: 3.76 ms with 64, 3.13 with 128, 3.15 with 160),
+  // longer ones leave too few blocks on an SM (3.30 with 224, 3.68 with 288).
+  int rows = out_h <= 96 ? (int)((out_h + 31) / 32 * 32) : 96;
+  for (int w = rows + 32; out_h > 96 && w <= RR_MAX_ROWS; w += 32)
+    if ((out_h + w - 1) / w * w <= (out_h + rows - 1) / rows * rows) rows = w;
   // largest raw tile of a block (rows and columns of the four-neighbour footprint)
   int maxr = 0, maxc = 0;
-  for (int64_t r0 = 0; r0 < out_h; r0 += RC_ROWS)
-    maxr = std::max(maxr, iy[std::min<int64_t>(r0 + RC_ROWS, out_h) - 1] + 2 - iy[r0]);
-  for (int64_t c0 = 0; c0 < out_w; c0 += RC_COLS)
-    maxc = std::max(maxc, ix[std::min<int64_t>(c0 + RC_COLS, out_w) - 1] + 2 - ix[c0]);
+  for (int64_t r0 = 0; r0 < out_h; r0 += rows)
+    maxr = std::max(maxr, iy[std::min<int64_t>(r0 + rows, out_h) - 1] + 2 - iy[r0]);
+  for (int64_t c0 = 0; c0 < out_w; c0 += RR_COLS)
+    maxc = std::max(maxc, ix[std::min<int64_t>(c0 + RR_COLS, out_w) - 1] + 2 - ix[c0]);
   const int es = dtype == MLF_DTYPE_U16 ? 2 : 4, vec = 16 / es;
   const int slot = ((maxr + 2 * vec - 2) / vec) * vec;
-  const size_t smem = 2 * (size_t)SF * maxc * slot * es;  // two chunk buffers
-  const bool staged = navg == 1 && reinterpret_cast<uintptr_t>(d_raw) % 16 == 0 && maxc <= 8 &&
-                      smem <= 112 * 1024 && (out_w + RC_COLS - 1) / RC_COLS <= 65535;
-  const dim3 block(RC_ROWS, RC_COLS);
+  const size_t smem = 2 * (size_t)RR_SF * maxc * slot * es;  // two stage buffers
+  const int64_t gx = (out_h + rows - 1) / rows, gy = (out_w + RR_COLS - 1) / RR_COLS;
+  const int64_t stages = (n_out + RR_SF - 1) / RR_SF;
+  // the gather takes averaged frames, raw buffers off the 16-byte grid and pitches whose tiles
+  // would leave fewer than two blocks on an SM
+  const bool staged = navg == 1 && reinterpret_cast<uintptr_t>(d_raw) % 16 == 0 && smem <= 112 * 1024 && gy <= 65535;
+  // calls that the 128 x 4 tiles of 16 frames took were limited to 65535 such stages: still refused
+  if (staged && n_out > (int64_t)16 * 65535) {
+    int rows4 = 0, cols4 = 0;
+    for (int64_t r0 = 0; r0 < out_h; r0 += 128)
+      rows4 = std::max(rows4, iy[std::min<int64_t>(r0 + 128, out_h) - 1] + 2 - iy[r0]);
+    for (int64_t c0 = 0; c0 < out_w; c0 += 4)
+      cols4 = std::max(cols4, ix[std::min<int64_t>(c0 + 4, out_w) - 1] + 2 - ix[c0]);
+    if (cols4 <= 8 && 32 * (size_t)cols4 * ((rows4 + 2 * vec - 2) / vec * vec) * es <= 112 * 1024)
+      return fail(MLF_ERR_UNSUPPORTED, "mlf_rectify_frames: more than 1048560 output frames");
+  }
+  DevBuf part;
   if (staged) {
-    const void* kf = dtype == MLF_DTYPE_U16 ? (const void*)k_rectify_staged<uint16_t> : (const void*)k_rectify_staged<float>;
-    MLF_TRY(allow_max_dyn_smem(kf));
-    const int64_t chunks = (n_out + SF - 1) / SF;
-    // frames whose starts differ by multiples of 16 bytes share the staged column offsets
-    const int same_align = ((fstep * fstride) % vec == 0) ? 1 : 0;
-    if (chunks > 65535) return fail(MLF_ERR_UNSUPPORTED, "mlf_rectify_frames: more than 1048560 output frames");
-    // blocks loop over frame chunks (prefetching the next one): enough z-slices for about
-    // sixteen waves of resident blocks (a short last wave), each slice walking its chunks
-    int dev = 0, nsm = 0;
-    MLF_CUDA(cudaGetDevice(&dev));
-    MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t gxy = ((out_h + RC_ROWS - 1) / RC_ROWS) * ((out_w + RC_COLS - 1) / RC_COLS);
-    const int64_t zb = std::max<int64_t>(1, std::min<int64_t>(chunks, (16 * 3 * (int64_t)nsm + gxy - 1) / gxy));
-    const dim3 grid((unsigned)((out_h + RC_ROWS - 1) / RC_ROWS), (unsigned)((out_w + RC_COLS - 1) / RC_COLS),
-                    (unsigned)zb);
+    RectifyRows A{};
+    A.total = total; A.fstride = fstride; A.cstride = cstride; A.row0 = row0; A.col0 = col0;
+    A.iy = d_iy; A.wy = d_wy; A.ix = d_ix; A.wx = d_wx;
+    A.oh = (int)out_h; A.ow = (int)out_w;
+    A.f0 = f0; A.fstep = fstep; A.n_out = n_out; A.slot = slot; A.maxc = maxc;
+    const bool same = (fstep * fstride) % vec == 0;  // frames share their 16-byte alignment
+    // enough z-slices for about sixteen waves of resident blocks (a short last wave), each
+    // walking its stages with the next one in flight
+    const int64_t gz = std::max<int64_t>(1, std::min<int64_t>({stages, (16 * 10 * (int64_t)nsm + gx * gy - 1) / (gx * gy), 65535}));
+    const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)gz), block(rows, 2);
+    if (!normalize) {
+      MLF_TRY(launch_rows<RR_PLAIN>(dtype, d_raw, A, same, grid, block, smem, d_out, st));
+    } else {
+      const int64_t nb = gx * gy * gz;
+      MLF_TRY(part.alloc(sizeof(float) * (nb + 1), "rectification max partials"));
+      A.max_part = part.as<float>() + 1;
+      A.mx = part.as<float>();
+      MLF_TRY(launch_rows<RR_MAX>(dtype, d_raw, A, same, grid, block, smem, d_out, st));
+      k_rc_max<<<1, 1024, 0, st>>>(A.max_part, nb, part.as<float>());
+      MLF_LAUNCHED();
+      MLF_TRY(launch_rows<RR_DIV>(dtype, d_raw, A, same, grid, block, smem, d_out, st));
+    }
+  } else {
+    const int64_t per_block = (int64_t)RC_FCH * RC_NCH;
+    const int64_t hx = (out_h + RC_ROWS - 1) / RC_ROWS, hy = (out_w + RC_COLS - 1) / RC_COLS;
+    const int64_t hz = (n_out + per_block - 1) / per_block;
+    if (hz > 65535 || hy > 65535)
+      return fail(MLF_ERR_UNSUPPORTED, "mlf_rectify_frames: too many output frames or columns for one launch");
+    const dim3 grid((unsigned)hx, (unsigned)hy, (unsigned)hz), block(RC_ROWS, RC_COLS);
+    float* max_part = nullptr;
+    if (normalize) {
+      MLF_TRY(part.alloc(sizeof(float) * (hx * hy * hz + 1), "rectification max partials"));
+      max_part = part.as<float>() + 1;
+    }
     if (dtype == MLF_DTYPE_U16)
-      k_rectify_staged<uint16_t><<<grid, block, smem, st>>>(static_cast<const uint16_t*>(d_raw), total, fstride,
-                                                            cstride, row0, col0, d_iy, d_wy, (int)out_h, d_ix, d_wx,
-                                                            (int)out_w, f0, fstep, n_out, slot, maxc, same_align,
-                                                            d_out);
-    else
-      k_rectify_staged<float><<<grid, block, smem, st>>>(static_cast<const float*>(d_raw), total, fstride, cstride,
-                                                         row0, col0, d_iy, d_wy, (int)out_h, d_ix, d_wx, (int)out_w,
-                                                         f0, fstep, n_out, slot, maxc, same_align, d_out);
-    MLF_LAUNCHED();
-  } else {
-  const int64_t per_block = (int64_t)RC_FCH * RC_NCH;
-  if ((n_out + per_block - 1) / per_block > 65535 || (out_w + RC_COLS - 1) / RC_COLS > 65535)
-    return fail(MLF_ERR_UNSUPPORTED, "mlf_rectify_frames: too many output frames or columns for one launch");
-  const dim3 grid((unsigned)((out_h + RC_ROWS - 1) / RC_ROWS), (unsigned)((out_w + RC_COLS - 1) / RC_COLS),
-                  (unsigned)((n_out + per_block - 1) / per_block));
-  if (dtype == MLF_DTYPE_U16)
-    k_rectify<uint16_t><<<grid, block, 0, st>>>(static_cast<const uint16_t*>(d_raw), fstride, cstride, row0, col0,
+      k_rectify<uint16_t><<<grid, block, 0, st>>>(static_cast<const uint16_t*>(d_raw), fstride, cstride, row0, col0,
                                                   d_iy, d_wy, (int)out_h, d_ix, d_wx, (int)out_w, f0, fstep, navg,
-                                                  flast, n_out, d_out);
-  else
-    k_rectify<float><<<grid, block, 0, st>>>(static_cast<const float*>(d_raw), fstride, cstride, row0, col0, d_iy,
+                                                  flast, n_out, d_out, max_part);
+    else
+      k_rectify<float><<<grid, block, 0, st>>>(static_cast<const float*>(d_raw), fstride, cstride, row0, col0, d_iy,
                                                d_wy, (int)out_h, d_ix, d_wx, (int)out_w, f0, fstep, navg, flast, n_out,
-                                               d_out);
-  }
-  MLF_LAUNCHED();
-  if (normalize) {
-    constexpr int NB = 1024;
-    DevBuf part;
-    MLF_TRY(part.alloc(sizeof(float) * NB, "rectification max partials"));
-    k_rc_max<<<NB, 256, 0, st>>>(d_out, P * n_out, part.as<float>());
-    k_rc_scale<<<NB, 256, 0, st>>>(d_out, P * n_out, part.as<float>(), NB);
+                                               d_out, max_part);
     MLF_LAUNCHED();
-    MLF_CUDA(cudaStreamSynchronize(st));
-  } else {
-    MLF_CUDA(cudaStreamSynchronize(st));  // tables are released on return
+    if (normalize) {
+      const int64_t n = P * n_out;
+      k_rc_max<<<1, 1024, 0, st>>>(max_part, hx * hy * hz, part.as<float>());
+      const bool v4 = n % 4 == 0 && reinterpret_cast<uintptr_t>(d_out) % 16 == 0;
+      const int64_t want = ((v4 ? n / 4 : n) + 255) / 256;
+      const unsigned nb = (unsigned)std::min<int64_t>(want, 64 * (int64_t)nsm);
+      if (v4)
+        k_rc_scale<true><<<nb, 256, 0, st>>>(d_out, n, part.as<float>());
+      else
+        k_rc_scale<false><<<nb, 256, 0, st>>>(d_out, n, part.as<float>());
+      MLF_LAUNCHED();
+    }
   }
+  MLF_CUDA(cudaStreamSynchronize(st));  // the tables and partials are released on return
   return MLF_OK;
 }
 
