@@ -152,7 +152,8 @@ int mlf_summary_image(const float* movie, int64_t P, int64_t T, int32_t mode, in
                       float* bg_temporal_out, void* stream);
 /* The same, with the device time of each pass (CUDA events on `stream`) in pass_ms[5]:
  * first column pass (with the max), mean later column pass, mean row pass, last pass (the
- * image), finalisation (image max and scale); pass_ms may be NULL. */
+ * image), finalisation (image max and scale); pass_ms may be NULL.  Where row and column pass are
+ * one read of the movie, the row entry is that pass and the column entry the sum over its parts. */
 int mlf_summary_image_ex(const float* movie, int64_t P, int64_t T, int32_t mode, int32_t bg_iter,
                          int32_t window_1, int32_t window_2, int32_t poly_index, float* summary_out,
                          float* bg_spatial_out, float* bg_temporal_out, double* pass_ms, void* stream);

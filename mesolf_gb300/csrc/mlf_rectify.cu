@@ -25,6 +25,7 @@
 // 2 x 2 + 4 bytes per pixel of 16-bit frames where write, maximum and scaling passes moved 18.
 // Averaged frames read navg frames per output, so there the write pass takes the maximum and a
 // scaling pass follows (2 navg + 12 bytes).
+#include "mlf_f32x2.cuh"
 #include "mlf_internal.h"
 
 #include <algorithm>
@@ -153,33 +154,6 @@ enum RectifyMode { RR_PLAIN = 0, RR_MAX = 1, RR_DIV = 2 };
 __device__ __forceinline__ float rr_raw(uint16_t x) { return __uint_as_float(0x4B000000u | x); }
 __device__ __forceinline__ float rr_raw(float x) { return x; }
 
-using f32x2 = unsigned long long;  // two FP32 values (lower half: the thread's first frame)
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-  return d;
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
 __device__ __forceinline__ void rc_cp_async16(void* smem, const void* gmem, int src_bytes) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(src_bytes) : "memory");
@@ -261,7 +235,7 @@ k_rectify_rows(const TIn* __restrict__ raw, RectifyRows A, float* __restrict__ o
   const bool mine = r < A.oh;
   const int lr = mine ? __ldg(A.iy + r) - rlo : 0;
   const float fy = mine ? __ldg(A.wy + r) : 0.f;
-  const f32x2 fy2 = pack2(fy, fy), minus1 = pack2(-1.f, -1.f);
+  const f32x2 fy2 = pack2(fy, fy);
   const int64_t P = (int64_t)A.oh * A.ow;
   const int cs = (int)(A.cstride & (VEC - 1));
   float mx = MODE == RR_DIV ? __ldg(A.mx) : -INFINITY;
@@ -297,7 +271,7 @@ k_rectify_rows(const TIn* __restrict__ raw, RectifyRows A, float* __restrict__ o
         const int ob = SAME ? oa : k * A.slot + ((lb + k * cs) & (VEC - 1));
         const f32x2 x0 = pack2(rr_raw(pa[oa]), rr_raw(pb[ob])), x1 = pack2(rr_raw(pa[oa + 1]), rr_raw(pb[ob + 1]));
         const f32x2 a = sizeof(TIn) == 2 ? add2(x0, pack2(-8388608.f, -8388608.f)) : x0;
-        return fma2(fma2(x0, minus1, x1), fy2, a);
+        return fma2(sub2(x1, x0), fy2, a);
       };
       float* op = out + r + (int64_t)A.oh * c0 + P * (ib + qa);
       f32x2 left = 0, right = 0;
@@ -311,7 +285,7 @@ k_rectify_rows(const TIn* __restrict__ raw, RectifyRows A, float* __restrict__ o
         if (t.x < 0) left = column(lc);  // block-uniform: a raw column was skipped or repeated
         right = column(lc + 1);
         const float fx = __int_as_float(t.y);
-        const f32x2 o2 = fma2(fma2(left, minus1, right), pack2(fx, fx), left);
+        const f32x2 o2 = fma2(sub2(right, left), pack2(fx, fx), left);
         if (MODE == RR_MAX) {
           const float2 o = unpack2(o2);
           mx = fmaxf(mx, fmaxf(o.x, o.y));

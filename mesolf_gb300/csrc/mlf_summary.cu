@@ -13,9 +13,11 @@
 //                 B = mean(y), C = mean(t) (compute_std_image as written)
 //   summary = img / max(img).
 //
-// Passes over the movie (HBM-bound streams): one column pass per iteration (the first also
-// takes the max), one row pass per iteration but the last, and a last row pass that also
-// computes the image.  bg_iter = 5 reads the movie 2 * bg_iter times.
+// Passes over the movie (HBM-bound streams): a first column pass (t = colsum, and the max), then
+// one pass per iteration but the last that forms s and the next t together (k_si_power), and a
+// last row pass that also computes the image: bg_iter = 5 reads the movie 6 times.  Movies that
+// k_si_power does not take (more than 2048 frames, off the 16-byte grid) need a row and a
+// column pass per iteration, 2 * bg_iter reads.
 //
 // Column passes: one block per 4 frames x pixel split; each float4 of s is loaded once for
 // the 4 frames; partial sums per split are reduced in a fixed order (deterministic).  Row
@@ -23,6 +25,8 @@
 // register prefetch of the next group of frames.  The moving means run as sliding window
 // sums over ring buffers in shared memory (one ring column per thread, conflict-free); the
 // window-1 sum carries a TwoSum compensation term so that its error does not grow with T.
+#include <cooperative_groups.h>
+
 #include "mlf_internal.h"
 
 namespace mlf {
@@ -121,36 +125,57 @@ k_si_coldot(const float* __restrict__ Y, int64_t P, int64_t T, const float* __re
 
 // One block: t = sum over splits of t_part (fixed order), t /= |t| (FP64 norm), mean(t);
 // nmax > 0: M = max(max_part[0..nmax)).
+// Bound: latency of the one block, and FP64, of which an SM does two operations a cycle: so four
+// warps take the two FP64 sums (32 warps' shuffles alone cost 2 x 1.3 us) and the division by the
+// norm is one reciprocal.
 __global__ void __launch_bounds__(SI_RED_THREADS)
 k_si_tnorm(const float* __restrict__ t_part, int ps, int64_t T, const float* __restrict__ max_part, int64_t nmax,
            float* __restrict__ t, float* __restrict__ scal) {
-  __shared__ double shd[32];
+  constexpr int NS = 128;  // threads of the FP64 sums
+  __shared__ double shd[2][NS / 32];
   __shared__ float shf[32];
-  __shared__ double bc[2];
-  double ss = 0.0;
-  for (int64_t j = threadIdx.x; j < T; j += SI_RED_THREADS) {
+  const int tid = threadIdx.x;
+  for (int64_t j = tid; j < T; j += SI_RED_THREADS) {
     float v = 0.f;
-    for (int s = 0; s < ps; ++s) v += t_part[(int64_t)s * T + j];
+    for (int s0 = 0; s0 < ps; s0 += 16) {  // 16 splits' loads in flight, added in order
+      float x[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) x[u] = t_part[(int64_t)min(s0 + u, ps - 1) * T + j];
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (s0 + u < ps) v += x[u];
+    }
     t[j] = v;
-    ss += (double)v * v;
   }
-  ss = block_sum(ss, shd);
-  if (threadIdx.x == 0) bc[0] = sqrt(ss);
   __syncthreads();
-  const double nrm = bc[0];
-  double st = 0.0;
-  for (int64_t j = threadIdx.x; j < T; j += SI_RED_THREADS) {
-    const float v = (float)((double)t[j] / nrm);
-    t[j] = v;
-    st += v;
+  if (tid < NS) {
+    double ss = 0.0, st = 0.0;
+    for (int64_t j = tid; j < T; j += NS) {
+      const double v = t[j];
+      ss += v * v;
+      st += v;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      ss += __shfl_down_sync(0xffffffffu, ss, o);
+      st += __shfl_down_sync(0xffffffffu, st, o);
+    }
+    if ((tid & 31) == 0) {
+      shd[0][tid >> 5] = ss;
+      shd[1][tid >> 5] = st;
+    }
   }
-  st = block_sum(st, shd);
-  if (threadIdx.x == 0) scal[SC_TMEAN] = (float)(st / (double)T);
+  __shared__ double rn;
+  __syncthreads();
+  if (tid == 0) rn = 1.0 / sqrt((shd[0][0] + shd[0][1]) + (shd[0][2] + shd[0][3]));
+  __syncthreads();
+  const double rnrm = rn;
+  for (int64_t j = tid; j < T; j += SI_RED_THREADS) t[j] = (float)((double)t[j] * rnrm);
+  if (tid == 0) scal[SC_TMEAN] = (float)(((shd[1][0] + shd[1][1]) + (shd[1][2] + shd[1][3])) * rnrm / (double)T);
   if (nmax > 0) {
     float m = -INFINITY;
-    for (int64_t i = threadIdx.x; i < nmax; i += SI_RED_THREADS) m = fmaxf(m, max_part[i]);
+    for (int64_t i = tid; i < nmax; i += SI_RED_THREADS) m = fmaxf(m, max_part[i]);
     m = block_max(m, shf);
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
       scal[SC_M] = m;
       scal[SC_INVM] = 1.f / m;
     }
@@ -210,6 +235,173 @@ k_si_rowdot1(const float* __restrict__ Y, int64_t P, int64_t T, const float* __r
   }
   for (; j < T; ++j) a = fmaf(__ldcs(y + j * P), __ldg(t + j), a);
   s[p] = (a + b) * scal[SC_INVM];
+}
+
+// One power iteration in one read of the movie: s = Y t / M and t_part = Y' s, t_part summed over
+// clusters by k_si_tnorm.  A cluster of up to 8 CTAs splits the frames (rows per CTA <= SP_ROWS)
+// and walks blocks of PB pixels.  Per block a CTA takes its rows x PB tile from shared memory into
+// registers (32 values per thread), forms its part of s, adds the parts of the cluster's CTAs
+// through distributed shared memory, and multiplies the same registers by s into its frames' t,
+// accumulated in registers over all its blocks.
+//
+// Bound: HBM, at the rate that 256-byte pieces of rows a frame apart give (4.1 TB/s with 2000
+// frames of 4 MB, 4.9 with 500 frames of 0.8 MB).  The two-pass form reads the movie once for s and
+// once for t, at 6.4 and 5.7 TB/s; this reads it once: 1.97 ms against 1.26 + 1.41 at
+// 1005 x 1005 x 2000, 0.83 against 1.36 with 1000 frames, 85 us against 66 + 86 at 465 x 450 x 500.
+// With more than 8 x 256 frames (32-pixel pieces: 4.3 against 4.0 ms at 1005 x 1005 x 3000) the two
+// passes stay.  The tile of the block in work is in registers, so all three 68 KB stages are in
+// flight.  The threads that publish s copy nothing: the release of a cluster barrier waits for the
+// thread's own outstanding accesses.
+//
+// Layout: row r holds the 16-byte vectors that cover its PB pixels (PB + 4 floats); pixel p is at
+// o + p with o = (frame * P) mod 4.  The rows of a thread are a multiple of 4 apart, so its o is
+// one value.  Y is 16-byte aligned; bytes past the movie's end are zero-filled, not read.
+constexpr int SP_THREADS = 512, SP_STAGES = 3;
+constexpr int SP_PB = 64, SP_RT = 32;              // pixels per block, rows per thread
+constexpr int SP_ROWS = SP_RT * SP_THREADS / SP_PB;  // 256 frames per CTA at most
+constexpr int SP_MAX_CLUSTER = 8;
+
+__device__ __forceinline__ void si_cp_async16(float* smem, const float* gmem, int src_bytes) {
+  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(src_bytes) : "memory");
+}
+
+__global__ void __launch_bounds__(SP_THREADS, 1)
+k_si_power(const float* __restrict__ Y, int64_t P, int64_t T, int rows, const float* __restrict__ t,
+           const float* __restrict__ scal, float* __restrict__ t_part) {
+  namespace cg = cooperative_groups;
+  constexpr int PB = SP_PB, NT = SP_THREADS;
+  constexpr int G = NT / PB;  // thread (pixel pa, group ga) owns rows ga, ga + G, ...
+  constexpr int SLOT = PB + 4, NV = SLOT / 4;
+  static_assert(G % 4 == 0, "a thread's rows must share their alignment");
+  extern __shared__ __align__(16) float tiles[];  // [SP_STAGES][rows][SLOT]
+  __shared__ __align__(16) float ts[G][SP_RT];    // t of row ga + G k at [ga][k], 0 past the last frame
+  __shared__ float red[G][PB], sbuf[2][PB], stot[PB];
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int tid = threadIdx.x;
+  const int64_t j0 = (int64_t)rank * rows;
+  const int nr = (int)max((int64_t)0, min((int64_t)rows, T - j0));  // frames of this CTA
+  const int64_t total = P * T, blocks = (P + PB - 1) / PB;
+  const int64_t first = blockIdx.x / C, ncl = gridDim.x / C;  // the host launches at most `blocks` clusters
+  const int n = (int)((blocks - first + ncl - 1) / ncl);      // blocks of this cluster
+  const int stage_floats = rows * SLOT;
+
+  // Vector e of a stage (row e / NV) goes to floats 4e; threads PB.. copy e = le, le + NL, ...
+  constexpr int NL = NT - PB, RV = (SP_ROWS * NV + NL - 1) / NL;
+  const int le = tid - PB;
+  const int64_t base = (j0 * P) & ~(int64_t)3;
+  uint32_t rel[RV];  // first element of each vector for pixel 0, from `base` (rows * P < 2^32: host)
+#pragma unroll
+  for (int k = 0; k < RV; ++k) {
+    const int e = max(le, 0) + NL * k, r = e / NV;
+    rel[k] = (uint32_t)((((j0 + r) * P) & ~(int64_t)3) - base) + 4 * (e - r * NV);
+  }
+  auto load = [&](int i) {
+    if (i < n && le >= 0) {
+      float* dst = tiles + (i % SP_STAGES) * stage_floats + 4 * le;
+      const int64_t p0 = (first + i * ncl) * PB;
+      const float* src = Y + base + p0;
+      if (p0 + PB + 4 <= P) {
+#pragma unroll
+        for (int k = 0; k < RV; ++k)
+          if (le + NL * k < nr * NV) si_cp_async16(dst + 4 * NL * k, src + rel[k], 16);
+      } else {  // the movie may end inside the last vectors of its last frame
+        for (int e = le; e < nr * NV; e += NL) {
+          const int r = e / NV;
+          const int64_t at = (((j0 + r) * P) & ~(int64_t)3) + 4 * (e - r * NV) + p0, avail = total - at;
+          const int bytes = avail >= 4 ? 16 : (avail > 0 ? 4 * (int)avail : 0);
+          si_cp_async16(dst + 4 * (e - le), bytes > 0 ? Y + at : Y, bytes);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  for (int i = 0; i < SP_STAGES; ++i) load(i);
+  for (int e = tid; e < G * SP_RT; e += NT) {
+    const int row = e / SP_RT + G * (e % SP_RT);
+    ts[e / SP_RT][e % SP_RT] = row < nr ? __ldg(t + j0 + row) : 0.f;
+  }
+  const int pa = tid % PB, ga = tid / PB;
+  const int oa = (int)(((j0 + ga) * P) & 3);
+  const int nk = ga < nr ? (nr - ga + G - 1) / G : 0;  // rows of this thread
+  const float invM = scal[SC_INVM];
+  float acc[SP_RT];
+#pragma unroll
+  for (int k = 0; k < SP_RT; ++k) acc[k] = 0.f;
+
+  for (int i = 0; i < n; ++i) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(SP_STAGES - 1) : "memory");
+    __syncthreads();  // block i staged by every thread; red, sbuf and stot of block i - 1 are read
+    const float* src = tiles + (i % SP_STAGES) * stage_floats + ga * SLOT + oa + pa;
+    float y[SP_RT], a = 0.f, b = 0.f;
+#pragma unroll
+    for (int k = 0; k < SP_RT; ++k) y[k] = k < nk ? src[G * k * SLOT] : 0.f;
+#pragma unroll
+    for (int k = 0; k < SP_RT; k += 4) {
+      const float4 tk = *reinterpret_cast<const float4*>(&ts[ga][k]);
+      a = fmaf(y[k], tk.x, a);
+      b = fmaf(y[k + 1], tk.y, b);
+      a = fmaf(y[k + 2], tk.z, a);
+      b = fmaf(y[k + 3], tk.w, b);
+    }
+    red[ga][pa] = a + b;
+    __syncthreads();  // red complete; the stage is in registers
+    if (tid < PB) {
+      float v = 0.f;
+#pragma unroll
+      for (int g = 0; g < G; ++g) v += red[g][tid];
+      sbuf[i & 1][tid] = v;
+    }
+    if (C > 1) {
+      if (tid < PB)  // whole warps
+        asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      else
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;\n" ::: "memory");
+    }
+    load(i + SP_STAGES);
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    if (tid < PB) {
+      // sbuf[i & 1] is written again for block i + 2, after the barrier of block i + 1, at which
+      // every CTA has read it
+      float v = sbuf[i & 1][tid];  // one CTA: this thread's own value
+      if (C > 1) {
+        float part[SP_MAX_CLUSTER];
+#pragma unroll
+        for (int r = 0; r < SP_MAX_CLUSTER; ++r) part[r] = r < C ? *cl.map_shared_rank(&sbuf[i & 1][tid], r) : 0.f;
+        v = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
+      }
+      stot[tid] = v * invM;
+    }
+    __syncthreads();
+    if ((first + i * ncl) * PB + pa < P) {  // pixels past the last one contribute nothing
+      const float s = stot[pa];
+#pragma unroll
+      for (int k = 0; k < SP_RT; ++k) acc[k] = fmaf(y[k], s, acc[k]);
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+  // t of row ga + G k: the sums of the group's two warps
+  float* out = t_part + (blockIdx.x / C) * T + j0;
+  constexpr int HW = PB / 32;
+  static_assert(G * SP_RT * HW == G * PB, "the warp sums take red's place");
+  float* wsum = &red[0][0];  // [G][SP_RT][HW]
+#pragma unroll
+  for (int k = 0; k < SP_RT; ++k) {
+    float v = acc[k];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((tid & 31) == 0) wsum[(ga * SP_RT + k) * HW + pa / 32] = v;
+  }
+  __syncthreads();
+  for (int e = tid; e < G * SP_RT; e += NT) {
+    const int row = e / SP_RT + G * (e % SP_RT);
+    float v = wsum[e * HW];
+#pragma unroll
+    for (int h = 1; h < HW; ++h) v += wsum[e * HW + h];
+    if (row < nr) out[row] = v;
+  }
+  if (C > 1) cl.sync();  // no CTA leaves while its shared memory is read
 }
 
 template <int POLY>
@@ -473,6 +665,54 @@ int summary_block(int64_t T, int w1, int w2, size_t smem_max, size_t* smem) {
 }
 
 namespace {
+// One power iteration in one pass (k_si_power): CTAs per cluster, frames per CTA and clusters;
+// clusters = 0 where it does not apply (a movie off the 16-byte grid, more than 2048 frames).
+struct PowerPlan {
+  int cluster = 1, rows = 0, clusters = 0;
+};
+size_t power_smem(int64_t rows) { return sizeof(float) * SP_STAGES * (size_t)rows * (SP_PB + 4); }
+int power_fit(PowerPlan* pp, int64_t P, int64_t T) {
+  int c = 1;
+  while (c < SP_MAX_CLUSTER && cdiv(T, c) > SP_ROWS) c *= 2;
+  if (cdiv(T, c) > SP_ROWS || cdiv(T, c) * P >= ((int64_t)1 << 32)) return MLF_OK;
+  MLF_TRY(allow_max_dyn_smem((const void*)k_si_power));
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)c;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)c);
+  cfg.blockDim = dim3(SP_THREADS);
+  cfg.dynamicSmemBytes = power_smem(cdiv(T, c));
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int nc = 0;
+  MLF_CUDA(cudaOccupancyMaxActiveClusters(&nc, k_si_power, &cfg));
+  if (nc < 1) return MLF_OK;
+  pp->cluster = c;
+  pp->rows = (int)cdiv(T, c);
+  pp->clusters = (int)std::min<int64_t>(nc, cdiv(P, SP_PB));
+  return MLF_OK;
+}
+int power_launch(const PowerPlan& pp, const float* Y, int64_t P, int64_t T, const float* t, const float* scal,
+                 float* t_part, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)pp.cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(pp.cluster * pp.clusters));
+  cfg.blockDim = dim3(SP_THREADS);
+  cfg.dynamicSmemBytes = power_smem(pp.rows);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  MLF_CUDA(cudaLaunchKernelEx(&cfg, k_si_power, Y, P, T, pp.rows, t, scal, t_part));
+  return MLF_OK;
+}
+}  // namespace
+
+namespace {
 // CUDA events around each pass when pass times are wanted (none otherwise)
 struct PassClock {
   std::vector<cudaEvent_t> ev;
@@ -517,41 +757,50 @@ int summary_run(const float* dY, int64_t P, int64_t T, int mode, int bg_iter, in
   int64_t ps = std::max<int64_t>(1, std::min<int64_t>(cdiv(2432, ngrp), P / 16384));
   int64_t chunk = (cdiv(P, ps) + 3) / 4 * 4;
   ps = cdiv(P, chunk);
+  PowerPlan pp;
+  if (bg_iter > 1 && reinterpret_cast<uintptr_t>(dY) % 16 == 0) {
+    MLF_TRY(power_fit(&pp, P, T));
+  }
   const int64_t nrow = cdiv(P, nt);
-  DevBuf tpart, maxpart, scal, imgpart, sbuf, tbuf;
-  MLF_TRY(tbuf.alloc(sizeof(float) * (T + 4), "summary: temporal background"));  // 16-byte aligned
-  float* tb = tbuf.as<float>();
-  MLF_TRY(tpart.alloc(sizeof(float) * ps * T, "summary: column partial sums"));
-  MLF_TRY(maxpart.alloc(sizeof(float) * ps * ngrp, "summary: max partials"));
-  MLF_TRY(scal.alloc(sizeof(float) * SC_N, "summary: scalars"));
-  MLF_TRY(imgpart.alloc(sizeof(float) * std::max(nrow, cdiv(P, SI_ROW_THREADS)), "summary: image max partials"));
-  MLF_TRY(sbuf.alloc(sizeof(float) * P, "summary: spatial background"));
-  float* sc = scal.as<float>();
+  // one allocation for the scratch (each costs a call and, at its release, a device
+  // synchronisation), every part 16-byte aligned
+  const int64_t parts[6] = {T + 4, std::max<int64_t>(ps, pp.clusters) * T, ps * ngrp, SC_N,
+                            std::max(nrow, cdiv(P, SI_ROW_THREADS)), P};
+  int64_t off[7] = {0};
+  for (int k = 0; k < 6; ++k) off[k + 1] = off[k] + (parts[k] + 3) / 4 * 4;
+  DevBuf scratch;
+  MLF_TRY(scratch.alloc(sizeof(float) * off[6], "summary: scratch"));
+  float* const tb = scratch.as<float>();
+  float* const tpart = tb + off[1];
+  float* const maxpart = tb + off[2];
+  float* const sc = tb + off[3];
+  float* const imgpart = tb + off[4];
+  float* const s_tmp = tb + off[5];
   const dim3 cgrid((unsigned)ngrp, (unsigned)ps);
-  float* s_tmp = sbuf.as<float>();
-  const bool s_aligned = reinterpret_cast<uintptr_t>(s_tmp) % 16 == 0;
   MLF_TRY(clk.mark(st));
   for (int it = 0; it < bg_iter; ++it) {
     if (it == 0) {
       if (vec)
-        k_si_coldot<true, true><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, nullptr, chunk, tpart.as<float>(),
-                                                                  maxpart.as<float>());
+        k_si_coldot<true, true><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, nullptr, chunk, tpart,
+                                                                  maxpart);
       else
-        k_si_coldot<false, true><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, nullptr, chunk, tpart.as<float>(),
-                                                                   maxpart.as<float>());
-    } else {
-      if (vec && s_aligned)
-        k_si_coldot<true, false><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, s_tmp, chunk, tpart.as<float>(), nullptr);
+        k_si_coldot<false, true><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, nullptr, chunk, tpart,
+                                                                   maxpart);
+    } else if (pp.clusters == 0) {
+      if (vec)
+        k_si_coldot<true, false><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, s_tmp, chunk, tpart, nullptr);
       else
-        k_si_coldot<false, false><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, s_tmp, chunk, tpart.as<float>(), nullptr);
+        k_si_coldot<false, false><<<cgrid, SI_COL_THREADS, 0, st>>>(dY, P, T, s_tmp, chunk, tpart, nullptr);
     }
     MLF_LAUNCHED();
-    k_si_tnorm<<<1, SI_RED_THREADS, 0, st>>>(tpart.as<float>(), (int)ps, T, maxpart.as<float>(),
+    k_si_tnorm<<<1, SI_RED_THREADS, 0, st>>>(tpart, it > 0 && pp.clusters ? pp.clusters : (int)ps, T, maxpart,
                                              it == 0 ? ps * ngrp : 0, tb, sc);
     MLF_LAUNCHED();
     MLF_TRY(clk.mark(st));
     if (it + 1 < bg_iter) {
-      if (vec)
+      if (pp.clusters)  // this iteration's s and the next one's t
+        MLF_TRY(power_launch(pp, dY, P, T, tb, sc, tpart, st));
+      else if (vec)
         k_si_rowdot4<<<(unsigned)cdiv(P / 4, SI_ROW_THREADS), SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, s_tmp);
       else
         k_si_rowdot1<<<(unsigned)cdiv(P, SI_ROW_THREADS), SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, s_tmp);
@@ -565,15 +814,15 @@ int summary_run(const float* dY, int64_t P, int64_t T, int mode, int bg_iter, in
     auto kp = poly == 1 ? k_si_pixelwise<1> : poly == 2 ? k_si_pixelwise<2> : poly == 3 ? k_si_pixelwise<3>
                                                                                       : k_si_pixelwise<-1>;
     MLF_TRY(allow_max_dyn_smem((const void*)kp));
-    kp<<<(unsigned)nrow, nt, smem, st>>>(dY, P, (int)T, tb, sc, w1, w2, R1, R2, poly, d_s, d_img, imgpart.as<float>());
+    kp<<<(unsigned)nrow, nt, smem, st>>>(dY, P, (int)T, tb, sc, w1, w2, R1, R2, poly, d_s, d_img, imgpart);
     nparts = nrow;
   } else {
     nparts = cdiv(P, SI_ROW_THREADS);
-    k_si_global<<<(unsigned)nparts, SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, d_s, d_img, imgpart.as<float>());
+    k_si_global<<<(unsigned)nparts, SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, d_s, d_img, imgpart);
   }
   MLF_LAUNCHED();
   MLF_TRY(clk.mark(st));
-  k_si_imgmax<<<1, SI_RED_THREADS, 0, st>>>(imgpart.as<float>(), nparts, sc);
+  k_si_imgmax<<<1, SI_RED_THREADS, 0, st>>>(imgpart, nparts, sc);
   k_si_scale<<<(unsigned)cdiv(P, 256), 256, 0, st>>>(d_img, P, sc);
   MLF_LAUNCHED();
   MLF_TRY(clk.mark(st));
