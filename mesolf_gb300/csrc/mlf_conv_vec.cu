@@ -9,20 +9,31 @@
 // (bitmap_end = x + kw/2 + 1) never reaches the last input column / row, so those are
 // treated as zero here too.
 //
-// Direct kernel (k_conv_vec_rows).  The outputs of one row phase b = y % 15 share one set
-// of 15 kernels (one per x phase), so a CTA takes rows y = b + 15 j of one slice and a
-// thread owns a segment of 15 consecutive outputs x = 15 i + a, a = 0..14 -- one per x
-// phase.  Per kernel row ky the CTA stages its input rows and the 15 kernels' row ky
-// ([kx][a], padded to 16) in shared memory with zero-filling cp.async, double buffered so
-// that row ky + 1 loads while row ky is computed.  Along kx the thread slides a window of
-// 15 inputs in registers (one new shared load per step) and reads the step's 15 taps as
-// broadcast 16-byte loads shared by the whole CTA; kw is padded to a multiple of 15 with
-// zero taps so that the 15-step rotation of the window needs no tail.  Every output still adds its products in
-// the reference's order -- kernel rows in order, each row left to right, one FP32 FMA chain
+// Direct kernel (k_conv_vec_lanes).  The outputs of one row phase b = y % 15 share one set of
+// 15 kernels (one per x phase).  A thread owns a segment of 15 consecutive outputs
+// x = 15 i + a, a = 0..14 -- one per x phase -- in RPT rows y = b + 15 j of one slice; the
+// (slice, row group, segment) triples of a phase are the lanes of its CTAs, so warps are full
+// whatever the sizes.  Per kernel row ky a CTA stages the input rows its lanes read and the 15
+// kernels' row ky ([kx][a], padded to 16) in shared memory with zero-filling cp.async, double
+// buffered so that row ky + 1 loads while row ky is computed.  Along kx the thread slides a window
+// of 15 inputs per row in registers (one new shared load per step and row) and reads the step's
+// 15 taps as broadcast 16-byte loads; kw is padded to a multiple of 15 with zero taps so that the
+// 15-step rotation of the window needs no tail.  Every output adds its products in the
+// reference's order -- kernel rows in order, each row left to right, one FP32 FMA chain
 // (mex_lfm_convolution_vec.cu:147-251) -- and the products it adds beyond the reference's
 // clipped window multiply zero-filled inputs, which adds exactly 0 for finite kernels; so
 // the output equals the reference kernel's bit for bit (tests/test_gpu_ref_mex.py).
+//
+// Bound: small calls have fewer warps than the chip has schedulers, so there one row per thread
+// spreads the work over the SMs; where the SMs are full, the shared-memory pipe, which returns a
+// step's taps to every warp (four 16-byte loads, 512 bytes each, for 15 FMAs per row): two rows
+// share them.  The columns that a row has off the image are zeroed once, so staging copies what
+// the image has and needs no test per element.  253 x 198 x 4, kw 136: 1.15 -> 0.60 ms (the
+// previous form launched 60 CTAs); 396 x 380 x 9, kw 151: 2.56 -> 2.07; 376 x 376 x 77, kw 241:
+// 45.2 -> 33.9 ms (37 TFLOP/s).
 #include <algorithm>
+#include <climits>
+#include <cmath>
 
 #include "mlf_internal.h"
 
@@ -30,139 +41,167 @@ namespace mlf {
 
 namespace {
 
-constexpr int CV_NN = 15;            // kernels per axis (the reference's num_kernels)
-constexpr int CV_MAX_THREADS = 768;  // rows a CTA's threads own at most (RPT rows per thread)
-constexpr int CV_RPT = 2;            // output rows per thread
+constexpr int CV_NN = 15;           // kernels per axis (the reference's num_kernels)
+constexpr int CV_MAX_THREADS = 384;  // 12 warps of up to 168 registers
+constexpr int CV_MAX_ROWS = 512;    // staged rows per CTA
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 4 : 0)
-               : "memory");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-struct ConvRowsArgs {
+struct ConvArgs {
   const float* in;   // W x H x n slices (x fastest)
   const float* K;    // kw x kw x 15 x 15 (kx fastest; kernel (a, b) at kw*kw*(a + 15 b))
   float* out;
   int W, H, kw, hk, Wv, Hv;  // Wv, Hv: columns / rows that can contribute (even kw: W-1, H-1)
   int kwp;                   // kw rounded up to a multiple of 15 (the extra taps are zero)
-  int sx, sy, tilesX;        // CTA tile: sx segments of 15 outputs x sy rows of one row phase
-  int width, pitch;          // staged input row: 15 sx + kw - 1 floats, pitch odd
-  int64_t slice0;            // first slice of this launch
+  int SX, tilesX;            // segments per group and groups along x
+  int width, pitch, gstride; // staged row: width = 15 SX + kwp - 1 floats, pitch apart; a group's RPT rows gstride
+  int max_groups;            // groups that a CTA's lanes can touch
+  int64_t n;                 // slices
 };
 
-// Stage input rows (row phase b, rows j0.., kernel row ky) and the 15 kernels' row ky into
-// buffer sel (zero where the reference reads nothing), then commit the copies.
-__device__ __forceinline__ void conv_rows_stage(const ConvRowsArgs& A, float* sm, float* rows0, int rowbuf,
-                                                const float* src, const float* kb, int64_t kplane, int b,
-                                                int j0, int nJ, int cstart, int ky, int sel) {
-  const int tid = threadIdx.x, nthr = blockDim.x;
-  float* rb = rows0 + sel * rowbuf;
-  // element e = r_l * width + c, advanced by nthr per step without a division
-  int r_l = tid / A.width, c = tid - r_l * A.width;
-  for (int e = tid; e < A.sy * A.width; e += nthr) {
-    const int r = b + CV_NN * (j0 + r_l) + ky - A.hk, col = cstart + c;
-    const bool ok = (j0 + r_l) < nJ && r >= 0 && r < A.Hv && col >= 0 && col < A.Wv;
-    cp_async4(rb + r_l * A.pitch + c, ok ? src + (int64_t)r * A.W + col : src, ok);
-    c += nthr;
-    while (c >= A.width) {
-      c -= A.width;
-      ++r_l;
-    }
-  }
-  float* tb = sm + sel * 16 * A.kwp;
-  const float* krow = kb + (int64_t)A.kw * ky;
-  for (int e = tid; e < 16 * A.kwp; e += nthr) {
-    const int kx = e >> 4, a = e & 15;
-    const bool ok = a < CV_NN && kx < A.kw;
-    cp_async4(tb + e, ok ? krow + kplane * a + kx : kb, ok);
-  }
-  cp_async_commit();
-}
-
-// RPT output rows per thread (rows jl*RPT .. jl*RPT + RPT-1 of the CTA's tile): the taps
-// of a step, loaded once, serve RPT rows.
+// Lane l of phase b: group l / SX = (slice * nP + row group) * tilesX + x tile, segment l % SX.
 template <int RPT>
-__global__ void __launch_bounds__(CV_MAX_THREADS / RPT, 1) k_conv_vec_rows(ConvRowsArgs A) {
+__global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
   extern __shared__ __align__(16) float sm[];
-  const int b = blockIdx.y;                      // row phase
-  const int64_t slice = A.slice0 + blockIdx.z;
-  const int i0 = (blockIdx.x % A.tilesX) * A.sx; // first segment
-  const int j0 = (blockIdx.x / A.tilesX) * A.sy; // first row index of phase b
-  const int nJ = b < A.H ? (A.H - b + CV_NN - 1) / CV_NN : 0;
-  if (j0 >= nJ) return;                           // CTA-uniform
-  const int tid = threadIdx.x;
-  const int il = tid % A.sx, jl = (tid / A.sx) * RPT;
-  const int x_seg = CV_NN * (i0 + il);
-  bool mine[RPT];
-  int yr[RPT];
-#pragma unroll
-  for (int r = 0; r < RPT; ++r) {
-    yr[r] = b + CV_NN * (j0 + jl + r);
-    mine[r] = jl + r < A.sy && x_seg < A.W && yr[r] < A.H;
+  __shared__ int row_y[CV_MAX_ROWS];          // staged row: image row at ky = 0 (INT_MIN / 2: none)
+  __shared__ int64_t row_src[CV_MAX_ROWS];    // ... its offset, at the tile's first column
+  __shared__ short2 row_col[CV_MAX_ROWS];     // ... staged columns [x, y) that the image has
+  const int b = blockIdx.y;                   // row phase
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int nJ = b < A.H ? (A.H - b + CV_NN - 1) / CV_NN : 0;  // rows of this phase
+  const int nP = (nJ + RPT - 1) / RPT;
+  const int64_t lanes = A.n * nP * A.tilesX * A.SX;
+  const int64_t l0 = (int64_t)blockIdx.x * nthr;
+  if (l0 >= lanes) return;  // CTA-uniform
+  const int64_t lN = lanes < l0 + nthr ? lanes : l0 + nthr;
+  const int64_t g0 = l0 / A.SX;
+  const int ng = (int)((lN - 1) / A.SX - g0) + 1;  // <= max_groups
+  auto group = [&](int64_t g, int& jp, int& xt) {  // -> slice
+    xt = (int)(g % A.tilesX);
+    const int64_t q = g / A.tilesX;
+    jp = (int)(q % nP);
+    return q / nP;
+  };
+  for (int rr = tid; rr < ng * RPT; rr += nthr) {
+    int jp, xt;
+    const int64_t slice = group(g0 + rr / RPT, jp, xt);
+    const int j = jp * RPT + rr % RPT;
+    const int y0 = b + CV_NN * j - A.hk;
+    row_y[rr] = j < nJ ? y0 : INT_MIN / 2;
+    const int c0 = CV_NN * A.SX * xt - A.hk;
+    const int ca = min(max(-c0, 0), A.width), cb = max(min(A.Wv - c0, A.width), ca);
+    row_col[rr] = make_short2((short)ca, (short)cb);
+    row_src[rr] = slice * (int64_t)A.W * A.H + (int64_t)y0 * A.W + c0;
   }
-  const int cstart = CV_NN * i0 - A.hk;          // input column of staged column 0
-  // taps first (16-byte aligned for the float4 loads), then the two row buffers
-  const int rowbuf = A.sy * A.pitch;
-  float* const rows0 = sm + 32 * A.kwp;  // buffer sel: taps sm + sel*16*kwp, rows rows0 + sel*rowbuf
-  const float* src = A.in + slice * (int64_t)A.W * A.H;
+  // this thread's lane
+  const int64_t lane_id = l0 + tid;
+  const bool active = lane_id < lanes;
+  const int64_t g = active ? lane_id / A.SX : g0;
+  const int il = active ? (int)(lane_id - g * A.SX) : 0;
+  int jp, xt;
+  const int64_t slice = group(g, jp, xt);
+  const int x_seg = CV_NN * (xt * A.SX + il);
+  const int rowbuf = A.max_groups * A.gstride;
+  float* const rows0 = sm + 32 * A.kwp;  // taps of buffer s at sm + 16 kwp s, rows at rows0 + rowbuf s
   const int64_t kplane = (int64_t)A.kw * A.kw;
-  const float* kb = A.K + kplane * CV_NN * b;    // kernels (a, b), a = 0..14
+  const float* kb = A.K + kplane * CV_NN * b;  // kernels (a, b), a = 0..14
+
+  // Kernel row ky into buffer s, then commit.  Columns off the image stay as zeroed below; a row
+  // off the image is zeroed where the buffer may hold another one.
+  const int warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
+  auto stage = [&](int ky, int s) {
+    float* tb = sm + s * 16 * A.kwp;
+    const int ta = tid & 15;
+    if (ta < CV_NN) {
+      const float* src = kb + kplane * ta + (int64_t)A.kw * ky;
+#pragma unroll 4
+      for (int kx = tid >> 4; kx < A.kw; kx += nthr >> 4) cp_async4(tb + 16 * kx + ta, src + kx);
+    }
+    float* rb = rows0 + s * rowbuf;
+    for (int rr = warp; rr < ng * RPT; rr += nwarps) {
+      const int y = row_y[rr] + ky;
+      const short2 cc = row_col[rr];
+      float* dst = rb + (rr / RPT) * A.gstride + (rr % RPT) * A.pitch;
+      if (y >= 0 && y < A.Hv) {
+        const float* src = A.in + row_src[rr] + (int64_t)ky * A.W;
+#pragma unroll 4
+        for (int c = cc.x + lane; c < cc.y; c += 32) cp_async4(dst + c, src + c);
+      } else {
+        for (int c = cc.x + lane; c < cc.y; c += 32) dst[c] = 0.f;
+      }
+    }
+    cp_async_commit();
+  };
+  // the padding taps are zero in both buffers; nothing writes them again
+  for (int e = tid; e < 2 * 16 * (A.kwp - A.kw); e += nthr) {
+    const int s = e / (16 * (A.kwp - A.kw)), k = e - s * 16 * (A.kwp - A.kw);
+    sm[s * 16 * A.kwp + 16 * A.kw + k] = 0.f;
+  }
+  for (int e = tid; e < 2 * rowbuf; e += nthr) rows0[e] = 0.f;
+  __syncthreads();  // the row table; the zeroed buffers
 
   float acc[RPT][CV_NN];
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
     for (int a = 0; a < CV_NN; ++a) acc[r][a] = 0.f;
-  conv_rows_stage(A, sm, rows0, rowbuf, src, kb, kplane, b, j0, nJ, cstart, 0, 0);
+  stage(0, 0);
   cp_async_wait0();
   __syncthreads();
   for (int ky = 0; ky < A.kw; ++ky) {
     const int sel = ky & 1;
-    if (ky + 1 < A.kw) conv_rows_stage(A, sm, rows0, rowbuf, src, kb, kplane, b, j0, nJ, cstart, ky + 1, sel ^ 1);
-    if (mine[0]) {
-      // rows past the tile read staged rows that exist (jl + r < sy is not required for the
-      // read: the buffer holds sy rows, so clamp) and are not stored
-      const float* rowp[RPT];
-#pragma unroll
-      for (int r = 0; r < RPT; ++r) rowp[r] = rows0 + sel * rowbuf + min(jl + r, A.sy - 1) * A.pitch + CV_NN * il;
+    if (ky + 1 < A.kw) stage(ky + 1, sel ^ 1);
+    if (active) {
+      const float* rowp = rows0 + sel * rowbuf + (int)(g - g0) * A.gstride + CV_NN * il;
       const float* tp = sm + sel * 16 * A.kwp;
-      float w[RPT][CV_NN];  // w[r][(m + a) % 15] holds rowp[r][kx0 + m + a]
+      float w[RPT][CV_NN];  // w[r][(m + a) % 15] holds row r at kx0 + m + a
 #pragma unroll
       for (int r = 0; r < RPT; ++r)
 #pragma unroll
-        for (int a = 0; a < CV_NN - 1; ++a) w[r][a] = rowp[r][a];
+        for (int a = 0; a < CV_NN - 1; ++a) w[r][a] = rowp[r * A.pitch + a];
+      const float4* t4 = reinterpret_cast<const float4*>(tp);
+      float4 tc[4];  // taps of the step in work; the next step's load during it
+#pragma unroll
+      for (int q = 0; q < 4; ++q) tc[q] = t4[q];
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) w[r][CV_NN - 1] = rowp[r * A.pitch + CV_NN - 1];
+#pragma unroll 1
       for (int kx0 = 0; kx0 < A.kwp; kx0 += CV_NN) {
 #pragma unroll
         for (int m = 0; m < CV_NN; ++m) {
+          float4 tn[4];
 #pragma unroll
-          for (int r = 0; r < RPT; ++r) w[r][(m + CV_NN - 1) % CV_NN] = rowp[r][kx0 + m + CV_NN - 1];
-          const float4* t4 = reinterpret_cast<const float4*>(tp + 16 * (kx0 + m));
-          float t[16];
+          for (int q = 0; q < 4; ++q) tn[q] = t4[4 * (kx0 + m + 1) + q];  // past the last step: not used
+          float wn[RPT];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 v = t4[q];
-            t[4 * q] = v.x;
-            t[4 * q + 1] = v.y;
-            t[4 * q + 2] = v.z;
-            t[4 * q + 3] = v.w;
-          }
+          for (int r = 0; r < RPT; ++r) wn[r] = rowp[r * A.pitch + kx0 + m + CV_NN];
+          const float t[16] = {tc[0].x, tc[0].y, tc[0].z, tc[0].w, tc[1].x, tc[1].y, tc[1].z, tc[1].w,
+                               tc[2].x, tc[2].y, tc[2].z, tc[2].w, tc[3].x, tc[3].y, tc[3].z, tc[3].w};
 #pragma unroll
-          for (int r = 0; r < RPT; ++r)
+          for (int a = 0; a < CV_NN; ++a)
 #pragma unroll
-            for (int a = 0; a < CV_NN; ++a) acc[r][a] = fmaf(w[r][(m + a) % CV_NN], t[a], acc[r][a]);
+            for (int r = 0; r < RPT; ++r) acc[r][a] = fmaf(w[r][(m + a) % CV_NN], t[a], acc[r][a]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) tc[q] = tn[q];
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) w[r][m] = wn[r];
         }
       }
     }
     cp_async_wait0();
     __syncthreads();
   }
+  if (!active) return;
 #pragma unroll
   for (int r = 0; r < RPT; ++r) {
-    if (!mine[r]) continue;
-    float* o = A.out + slice * (int64_t)A.W * A.H + (int64_t)yr[r] * A.W;
+    const int j = jp * RPT + r;
+    if (j >= nJ) continue;
+    float* o = A.out + slice * (int64_t)A.W * A.H + (int64_t)(b + CV_NN * j) * A.W;
 #pragma unroll
     for (int a = 0; a < CV_NN; ++a)
       if (x_seg + a < A.W) o[x_seg + a] = acc[r][a];
@@ -256,40 +295,88 @@ int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const f
   if (nnum != CV_NN) return fail(MLF_ERR_INVALID, "direct MEX projector: the kernel grid must be 15 x 15");
   if (W > (1 << 24) || H > (1 << 24) || W * H > ((int64_t)1 << 31))
     return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: slice larger than 2^31 pixels");
-  int dev = 0, optin = 0;
+  int dev = 0, optin = 0, nsm = 0;
   MLF_CUDA(cudaGetDevice(&dev));
   MLF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  MLF_TRY(allow_max_dyn_smem((const void*)k_conv_vec_rows<CV_RPT>));
-  ConvRowsArgs a{};
+  MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  ConvArgs a{};
   a.in = d_bitmap;
   a.K = d_kernels;
   a.out = d_out;
   a.W = (int)W;
   a.H = (int)H;
+  a.n = n;
   a.kw = (int)kw;
   a.hk = (int)(kw / 2);
   a.kwp = (a.kw + CV_NN - 1) / CV_NN * CV_NN;
   a.Wv = (kw % 2 == 0) ? a.W - 1 : a.W;  // even kw: the reference's clip never reaches the last column / row
   a.Hv = (kw % 2 == 0) ? a.H - 1 : a.H;
   const int nI = (a.W + CV_NN - 1) / CV_NN, nJ = (a.H + CV_NN - 1) / CV_NN;
-  a.sx = std::min(nI, 32);
-  a.width = CV_NN * a.sx + a.kwp - 1;
-  a.pitch = a.width | 1;  // odd: rows of a warp fall on different banks
-  const size_t tap_bytes = sizeof(float) * 2 * 16 * (size_t)a.kwp;
-  const size_t budget = (size_t)optin - 1024;
-  a.sy = std::max(1, std::min(nJ, CV_RPT * (CV_MAX_THREADS / CV_RPT / a.sx)));
-  while (a.sy > 1 && sizeof(float) * 2 * (size_t)a.sy * a.pitch + tap_bytes > budget) --a.sy;
-  const size_t smem = sizeof(float) * 2 * (size_t)a.sy * a.pitch + tap_bytes;
-  if (smem > budget) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
-  a.tilesX = (nI + a.sx - 1) / a.sx;
-  const int tilesY = (nJ + a.sy - 1) / a.sy;
-  const int threads = (a.sx * ((a.sy + CV_RPT - 1) / CV_RPT) + 31) / 32 * 32;
-  for (int64_t s0 = 0; s0 < n; s0 += 65535) {
-    a.slice0 = s0;
-    const dim3 grid((unsigned)(a.tilesX * tilesY), CV_NN, (unsigned)std::min<int64_t>(65535, n - s0));
-    k_conv_vec_rows<CV_RPT><<<grid, threads, smem, st>>>(a);
-    MLF_LAUNCHED();
+  a.tilesX = (nI + 31) / 32;  // at most 32 segments of a row per group, evenly
+  a.SX = (nI + a.tilesX - 1) / a.tilesX;
+  a.width = CV_NN * a.SX + a.kwp - 1;
+  a.pitch = a.width;
+  auto lanes_of = [&](int rpt) { return n * ((nJ + rpt - 1) / rpt) * (int64_t)a.tilesX * a.SX; };
+  const size_t budget = (size_t)optin - 12 * 1024;  // the row table is static
+  int smem_sm = 0;
+  MLF_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  // shared memory and group geometry of CTAs of `warps` warps and rpt rows per thread
+  auto plan = [&](int rpt, int warps, ConvArgs& c) {
+    c.gstride = rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
+    while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
+    c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (lanes_of(rpt) + c.SX - 1) / c.SX);
+    const size_t bytes = sizeof(float) * (2 * 16 * (size_t)c.kwp + 2 * (size_t)c.max_groups * c.gstride);
+    return bytes <= budget && c.max_groups * rpt <= CV_MAX_ROWS ? bytes : (size_t)0;
+  };
+  // Rows per thread and warps per CTA: the pair with the fewest cycles per kernel column.  A step
+  // takes 60 (one row) or 84 cycles (two rows) while the SM has at most one warp per scheduler, and
+  // 12.2 or 14.5 cycles of the SM per warp beyond that (measured; four rows took 138 and 27, no
+  // better per row).  So one row for a few segments per SM (253 x 198 x 4, kw 136: 0.60 ms against
+  // 0.83 with two), two where the SMs are full (376 x 376 x 77, kw 241: 34 ms against 48), and the
+  // CTA size that leaves the shortest last wave.
+  int rpt = 0, warps = 0;
+  size_t smem = 0;
+  double best = 0;
+  for (int r : {1, 2}) {
+    const double lone = r == 1 ? 60 : 84, each = r == 1 ? 12.2 : 14.5;
+    const int regs = r == 1 ? 80 : 112;
+    const int64_t wp = (lanes_of(r) + 31) / 32;  // warps per phase
+    for (int k = 1; k <= CV_MAX_THREADS / 32; ++k) {
+      ConvArgs c = a;
+      const size_t bytes = plan(r, k, c);
+      if (!bytes) continue;
+      const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (regs * 32 * k)));
+      const int64_t ctas = CV_NN * ((wp + k - 1) / k);
+      const int64_t waves = (ctas + nsm * per_sm - 1) / (nsm * per_sm);
+      const int64_t on_sm = std::min<int64_t>(per_sm, (ctas + nsm - 1) / nsm);
+      // the busiest of four schedulers; each CTA stages taps and rows of its own, shared by its
+      // warps (idle ones too: 40 x 35 x 2, kw 21 has 18 lanes per phase and takes 90 us with two
+      // warps, 75 with six), whose barriers cost more the more there are
+      const int64_t w = k * on_sm <= 4 ? 4 : (k * on_sm + 3) / 4 * 4;
+      const double stage = 8.0 * (0.5 + (double)(c.max_groups * r) * c.width / (32.0 * a.kw)) / k;
+      const double cyc = (double)waves * (std::max(lone, each * (double)w) + (stage + 2.0) * (double)on_sm + 0.7 * k);
+      if (!rpt || cyc < best) {
+        best = cyc;
+        rpt = r;
+        warps = k;
+        smem = bytes;
+      }
+    }
   }
+  if (!rpt) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
+  plan(rpt, warps, a);
+  const int threads = 32 * warps;
+  const int64_t lanes = lanes_of(rpt);
+  const int64_t ctas = (lanes + threads - 1) / threads;
+  if (ctas > INT32_MAX) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: too many slices");
+  const void* kf = rpt == 1 ? (const void*)k_conv_vec_lanes<1> : (const void*)k_conv_vec_lanes<2>;
+  MLF_TRY(allow_max_dyn_smem(kf));
+  const dim3 grid((unsigned)ctas, CV_NN);
+  if (rpt == 1)
+    k_conv_vec_lanes<1><<<grid, threads, smem, st>>>(a);
+  else
+    k_conv_vec_lanes<2><<<grid, threads, smem, st>>>(a);
+  MLF_LAUNCHED();
   return MLF_OK;
 }
 
