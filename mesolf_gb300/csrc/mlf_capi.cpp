@@ -648,7 +648,8 @@ int mlf_batch_plan_bytes(const mlf_psf* psf, int32_t npatch, const int64_t* Xr, 
     members += (size_t)(Xr[k] * Xc[k] * nz[k] * 4 + 4096 * 8 + (int64_t)nz[k] * (Xr[k] + Xc[k]) * 4 +
                         6 * (int64_t)nz[k] * 4 + (2 * (int64_t)nz[k] * gmax + nz[k]) * 8);
   }
-  *bytes = (int64_t)(members + tc_work_plan_bytes(psf, li, lj, nsm));
+  const std::vector<int> vz0(z0, z0 + npatch), vnz(nz, nz + npatch);
+  *bytes = (int64_t)(members + tc_work_plan_bytes(psf, li, lj, vz0, vnz, nsm));
   return MLF_OK;
 }
 

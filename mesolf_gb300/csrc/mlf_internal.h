@@ -267,7 +267,8 @@ size_t tc_psf_bytes(const Psf* p);
 size_t tc_solver_bytes(const Solver* s);
 size_t tc_work_bytes(const TcSolverState* w);
 // device bytes tc_work_create would allocate for patches of Li[p] x Lj[p] lenslets (upper bound)
-size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std::vector<int>& Lj, int nsm);
+size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std::vector<int>& Lj,
+                          const std::vector<int>& z0, const std::vector<int>& nz, int nsm);
 int filter_run(Solver* s, cudaStream_t st);
 int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const float* d_kernels,
                  int64_t kw, int nnum, float* d_out, cudaStream_t st);

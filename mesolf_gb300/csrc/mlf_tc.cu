@@ -34,10 +34,15 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <map>
 #include <memory>
+#include <queue>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "mlf_internal.h"
@@ -549,12 +554,31 @@ k_tc_bwd(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtens
 }
 
 // ------------------------------------------------------------------ forward projection
+// Split s of a patch: the channel tiles [n_lo, n_hi) of the patch's own planes, cut evenly (a
+// split of the whole volume would leave patches with few planes most of their work in one split),
+// and the forward GEMM's K-steps [ks0, ks1) inside them.  Empty splits have n_lo == n_hi.
+struct SplitRange {
+  int n_lo, n_hi, ks0, ks1;
+};
+__host__ __device__ inline SplitRange split_range(int z0, int nz, int NN, int splits, int s, int KS) {
+  SplitRange r;
+  const int t0 = z0 * NN / BWD_BN, t1 = ((z0 + nz) * NN + BWD_BN - 1) / BWD_BN;
+  const int per = (t1 - t0 + splits - 1) / splits;
+  r.n_lo = t0 + s * per < t1 ? t0 + s * per : t1;
+  r.n_hi = r.n_lo + per < t1 ? r.n_lo + per : t1;
+  constexpr int H = BWD_BN / BK;  // K-steps per channel tile
+  const int klo = z0 * NN / BK, khi = ((z0 + nz) * NN + BK - 1) / BK;
+  r.ks0 = H * r.n_lo > klo ? H * r.n_lo : klo;
+  r.ks1 = H * r.n_hi < khi ? H * r.n_hi : khi;
+  if (r.ks1 > KS) r.ks1 = KS;
+  return r;
+}
 constexpr int FWD_MAX_STAGES = 4;
 struct TcFwdArgs {
   float* ypart;  // [split][NB][MP] (tap-major: col2im reads it coalesced)
   int* err;
   int stages;    // shared-memory ring depth (2..FWD_MAX_STAGES)
-  int MP, NB, NH, nparts, ks_per_split, KS, frow0;  // frow0 = view * NB
+  int MP, NB, NH, nparts, splits, KS, frow0;  // frow0 = view * NB
   int use_alo, use_blo;                             // activation / tap hi+lo splits
   const float* wview;      // per patch weight of the projected view (nullable: project all)
   const int* tile_patch;   // patch of each position tile
@@ -600,10 +624,8 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
   const int split = blockIdx.y;
   // this split's channel blocks, clipped to the patch's planes (an empty range writes zeros)
   const int* pq = a.pinfo + 8 * __ldg(a.tile_patch + blockIdx.x);
-  const int klo = __ldg(pq + 4) * a.NN / BK;
-  const int khi = ((__ldg(pq + 4) + __ldg(pq + 5)) * a.NN + BK - 1) / BK;
-  const int ks0 = max(split * a.ks_per_split, klo);
-  const int ks1 = min(min(a.KS, split * a.ks_per_split + a.ks_per_split), khi);
+  const SplitRange sr = split_range(__ldg(pq + 4), __ldg(pq + 5), a.NN, a.splits, split, a.KS);
+  const int ks0 = sr.ks0, ks1 = sr.ks1;
   const int tileB = a.NB * 128;  // NB rows x 128 bytes
   const int S = a.stages;
   const int offAl = TILE_A, offBh = FWD_XTILE, offBl = offBh + tileB;
@@ -764,7 +786,8 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
 // shared memory, so the volume is read and written once per view (k_tc_fwd re-reads it).
 // Work items are (position tile m, split s): the channel tiles of split s -- the split
 // boundaries of k_tc_fwd, so Y accumulates over the same K-steps in the same order (the
-// results are bit for bit those of k_tc_bwd + k_tc_fwd).  Per tile:
+// results are bit for bit those of k_tc_bwd + k_tc_fwd).  The items of a CTA come from a table
+// that the host balances over the CTAs (tc_items).  Per tile:
 //   producer:  the 5 AR / Wb stages of tile i, then the 1-2 Wf half stages of tile i-1
 //   MMA:       back projection of tile i into C[i & 1], then the forward of tile i-1 into Y
 //   epilogue:  update of tile i (as k_tc_bwd); after the I/O warp has stored the FP32 half
@@ -780,15 +803,24 @@ struct TcFusedArgs {
   TcBwdArgs b;
   float* ypart;        // [splits][NB][MP]
   const float* wview;  // per patch weight of the projected (next) view
-  int MP, NB, splits, ks_per_split, KS, frow0, ntiles;
+  int MP, NB, splits, KS, frow0;
+  const int* items;    // entry c + k * gridDim.x: k-th item of CTA c (m * splits + s), -1: none;
+                       // null: entry e is item e (one item per CTA: a load less on the way in)
 };
 
 struct FusedItem {
   int m, s, n_lo, n_hi, ks0, ks1, c0, c1;
   bool wcur, wnext;
 };
-__device__ __forceinline__ FusedItem fused_item(const TcFusedArgs& a, int item) {
+// entry e of the item table (an empty range for -1)
+__device__ __forceinline__ FusedItem fused_item(const TcFusedArgs& a, int e) {
   FusedItem f;
+  const int item = a.items ? __ldg(a.items + e) : e;
+  if (item < 0) {
+    f.m = f.s = f.n_lo = f.n_hi = f.ks0 = f.ks1 = f.c0 = f.c1 = 0;
+    f.wcur = f.wnext = false;
+    return f;
+  }
   f.m = item / a.splits;
   f.s = item - f.m * a.splits;
   const int pp = __ldg(a.b.tile_patch + f.m);
@@ -796,12 +828,11 @@ __device__ __forceinline__ FusedItem fused_item(const TcFusedArgs& a, int item) 
   const int z0 = __ldg(pi + 4), nz = __ldg(pi + 5);
   f.c0 = z0 * a.b.NN;                 // channel range of the patch (as bwd_skip)
   f.c1 = f.c0 + nz * a.b.NN;
-  const int klo = z0 * a.b.NN / BK;   // K-steps of the forward (as k_tc_fwd)
-  const int khi = ((z0 + nz) * a.b.NN + BK - 1) / BK;
-  f.ks0 = max(f.s * a.ks_per_split, klo);
-  f.ks1 = min(min(a.KS, f.s * a.ks_per_split + a.ks_per_split), khi);
-  f.n_lo = f.s * (a.ks_per_split / 2);
-  f.n_hi = min(a.ntiles, (f.s + 1) * (a.ks_per_split / 2));
+  const SplitRange sr = split_range(z0, nz, a.b.NN, a.splits, f.s, a.KS);  // as k_tc_fwd
+  f.ks0 = sr.ks0;
+  f.ks1 = sr.ks1;
+  f.n_lo = sr.n_lo;
+  f.n_hi = sr.n_hi;
   f.wcur = __ldg(a.b.wrow + pp) != 0.f;
   f.wnext = a.wview ? __ldg(a.wview + pp) != 0.f : true;
   return f;
@@ -1571,15 +1602,22 @@ struct TcPsfState {
 // patch padded to whole 128-position tiles), the FP32 volume X[ch][position] of every
 // patch, the BF16 operand buffers, the union view order and per-patch view weights.
 struct TcSolverState {
-  int P = 0, MP = 0, Zch = 0, splits = 1, ks_per_split = 0, KSF = 0, nsm = 0;
+  int P = 0, MP = 0, Zch = 0, splits = 1, KSF = 0, nsm = 0;
   float d_eps = 0.f;  // the members' variant (all the same)
   // launch configuration per precision: split-K count of the forward GEMM (the partials
   // buffer holds splits_max), its ring depth, the back projection's X buffers per half
   struct Tune {
-    int done = 0, tuned = 0, splits = 0, ksp = 0, fwd_stages = 0, xbufs = 0;
+    int done = 0, tuned = 0, splits = 0, fwd_stages = 0, xbufs = 0;
   };
   Tune tune[kPrecModes];
-  int splits_max = 1, splits_def = 1, ksp_def = 0;
+  int splits_max = 1, splits_def = 1;
+  // item tables of the fused view step by split count: entries and CTAs (tc_items)
+  struct Items {
+    DevBuf tab;
+    int n = 0, grid = 0;
+    bool identity = false;
+  };
+  std::map<int, Items> items;
   int fwd_stages = 0, xbufs = 0;  // in use (0: derive from shared memory)
   bool dtab_ok = false;  // every patch has >= 2q+2 lenslets per side: D from class tables
   std::vector<int> pos0, Li, Lj, LL, z0, nz;
@@ -1730,7 +1768,78 @@ size_t tc_work_bytes(const TcSolverState* t) {
 
 size_t tc_solver_bytes(const Solver* s) { return tc_work_bytes(s->tc); }
 
-size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std::vector<int>& Lj, int nsm) {
+namespace {
+// Fused view step: the makespan over `grid` CTAs of the items (position tile, split) of all
+// patches, longest first to the least loaded CTA (cost in microseconds), and the assignment.
+struct ItemCost {
+  double us;
+  int item;
+};
+double assign_items(std::vector<ItemCost> items, int grid, std::vector<std::vector<int>>* lists) {
+  std::stable_sort(items.begin(), items.end(), [](const ItemCost& a, const ItemCost& b) { return a.us > b.us; });
+  std::priority_queue<std::pair<double, int>, std::vector<std::pair<double, int>>, std::greater<>> load;
+  for (int c = 0; c < grid; ++c) load.push({0.0, c});
+  double most = 0;
+  for (const ItemCost& i : items) {
+    auto [us, c] = load.top();
+    load.pop();
+    if (lists) (*lists)[c].push_back(i.item);
+    most = std::max(most, us + i.us);
+    load.push({us + i.us, c});
+  }
+  return most;
+}
+std::vector<ItemCost> item_costs(int NN, int KB, int NB, const std::vector<int>& tiles, const std::vector<int>& z0,
+                                 const std::vector<int>& nz, int splits) {
+  const double tile = 2.3 + 1.2 * (KB / BK), drain = 2.0 + 0.012 * NB;  // measured: 8.3 us at KB 320, 5.9 at 192
+  std::vector<ItemCost> out;
+  int m = 0;
+  for (size_t p = 0; p < tiles.size(); ++p)
+    for (int k = 0; k < tiles[p]; ++k, ++m)
+      for (int s = 0; s < splits; ++s) {
+        const SplitRange r = split_range(z0[p], nz[p], NN, splits, s, INT_MAX);
+        out.push_back({drain + tile * (r.n_hi - r.n_lo), m * splits + s});
+      }
+  return out;
+}
+// Splits of the forward GEMM.  The fused view step's items are (position tile, split), so the split
+// count sets how evenly they fill the CTAs: the count with the shortest makespan plus the time
+// that summing the splits' partials takes (8 us + 0.8 us per MB).  One split per SM and position
+// tile, as before, left 56 of 152 CTAs without an item for 96 position tiles in one split (six
+// patches of 31-60 lenslets and 13-26 planes, K0 171: 272 us per view step).
+struct SplitPlan {
+  int def = 1, max = 1;
+};
+SplitPlan plan_splits(int NN, int KB, int NB, const std::vector<int>& Li, const std::vector<int>& Lj,
+                      const std::vector<int>& z0, const std::vector<int>& nz, int nsm) {
+  std::vector<int> tiles;
+  int mt = 0, most = 1;
+  for (size_t p = 0; p < Li.size(); ++p) {
+    tiles.push_back((Li[p] * Lj[p] + BM - 1) / BM);
+    mt += tiles.back();
+    const SplitRange r = split_range(z0[p], nz[p], NN, 1, 0, INT_MAX);
+    most = std::max(most, r.n_hi - r.n_lo);
+  }
+  SplitPlan sp;
+  sp.max = std::min(most, 2);
+  if (mt > 64 * nsm) return sp;  // tiles enough for any balance
+  double best = 0;
+  for (int s = 1; s <= std::min(most, std::max(8, 2 * nsm / std::max(1, mt))); ++s) {
+    if (s > 1 && (int64_t)mt * s > 64 * (int64_t)nsm) break;
+    const double us = assign_items(item_costs(NN, KB, NB, tiles, z0, nz, s), std::min(mt * s, nsm), nullptr) + 8.0 +
+                      0.8e-6 * s * (double)mt * BM * NB * 4;
+    if (s == 1 || us < best) {
+      best = us;
+      sp.def = s;
+    }
+  }
+  sp.max = std::min(most, 2 * sp.def);
+  return sp;
+}
+}  // namespace
+
+size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std::vector<int>& Lj,
+                          const std::vector<int>& z0, const std::vector<int>& nz, int nsm) {
   const int KB = rup((psf->T + 2) * (psf->T + 2), BK);
   const int TT = psf->T * psf->T;
   const int NB = rup(TT, 16) > 256 ? rup(TT, 32) : rup(TT, 16);
@@ -1740,15 +1849,11 @@ size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std:
     MP += rup(Li[p] * Lj[p], BM);
     tiles += rup(Li[p] * Lj[p], BM) / BM;
   }
-  const int KSF = (int)(CHP / BK);
-  const int mt = (int)(MP / BM);
-  int splits = std::max(1, std::min(KSF, nsm / std::max(1, mt)));
-  const int ksp = (KSF + splits - 1) / splits;
-  splits = (KSF + ksp - 1) / ksp;
+  const SplitPlan sp = plan_splits(psf->N * psf->N, rup((psf->T + 2) * (psf->T + 2), BK), NB, Li, Lj, z0, nz, nsm);
   const int64_t P = (int64_t)Li.size();
   return (size_t)(psf->nch * MP * 4 + (int64_t)psf->N * psf->N * MP * 4 + MP * 4 + tiles * 4 + 8 * P * 4 +
                   (int64_t)psf->N * psf->N * P * 4 + P * 4 + 4 * MP * KB * 2 + 16 +
-                  (int64_t)splits * MP * NB * 4 + 4 +
+                  (int64_t)sp.max * MP * NB * 4 + 4 +
                   // convergence monitor, allocated by the first solve that asks for stats
                   psf->nch * MP * 4 + (int64_t)kRelChangeBufDoubles * 8);
 }
@@ -1795,15 +1900,9 @@ int tc_work_create(Psf* psf, const std::vector<Solver*>& members, TcSolverState*
   }
   t->KSF = tp->CHP / BK;
   MLF_CUDA(cudaDeviceGetAttribute(&t->nsm, cudaDevAttrMultiProcessorCount, members[0]->device));
-  const int mt = t->MP / BM;
-  t->splits = std::max(1, std::min(t->KSF, t->nsm / std::max(1, mt)));
-  // even K-steps per split: a split then covers whole 128-channel tiles (the fused kernel's
-  // work items keep the forward GEMM's split boundaries)
-  t->ks_per_split = (((t->KSF + t->splits - 1) / t->splits) + 1) & ~1;
-  t->splits = (t->KSF + t->ks_per_split - 1) / t->ks_per_split;
-  t->splits_def = t->splits;
-  t->ksp_def = t->ks_per_split;
-  t->splits_max = std::min(t->KSF, 2 * t->splits);
+  const SplitPlan sp = plan_splits(psf->N * psf->N, tp->KB, tp->NB, t->Li, t->Lj, t->z0, t->nz, t->nsm);
+  t->splits = t->splits_def = sp.def;
+  t->splits_max = sp.max;
   const int64_t nch = psf->nch;
   MLF_TRY(t->X.alloc((size_t)nch * t->MP * 4, "tc volume (FP32)"));
   MLF_TRY(t->lfs.alloc((size_t)psf->N * psf->N * t->MP * 4, "tc sub-aperture images"));
@@ -1906,7 +2005,7 @@ int tc_fwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, cud
   a.NB = tp->NB;
   a.NH = tp->NH;
   a.nparts = tp->nparts;
-  a.ks_per_split = t->ks_per_split;
+  a.splits = t->splits;
   a.KS = t->KSF;
   a.frow0 = view * tp->NB;
   a.use_alo = alo;
@@ -2042,17 +2141,44 @@ int tc_bwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, con
 
 
 // The fused back projection + next forward applies to the BF16 modes with D from the class
-// tables, a forward taps tile of one MMA (N <= 256) and even split sizes; MLF_FUSED=0 keeps
-// the two kernels.
+// tables and a forward taps tile of one MMA (N <= 256); MLF_FUSED=0 keeps the two kernels.
 bool tc_fused_ok(const Psf* psf, const TcSolverState* t, int precision) {
   if (precision != MLF_PREC_BF16 && precision != MLF_PREC_BF16X2) return false;
   const TcPsfState* tp = psf->tc;
-  if (!t->dtab_ok || tp->nparts != 1 || tp->NB > 256 || t->ks_per_split % 2 != 0) return false;
+  if (!t->dtab_ok || tp->nparts != 1 || tp->NB > 256) return false;
   const char* env = std::getenv("MLF_FUSED");
   if (env && std::strcmp(env, "0") == 0) return false;
   int alo, blo;
   splits_of(precision, &alo, &blo);
   return !blo && 3 * (size_t)bwd_layout(alo, 0, false).stage + XTILE + 1024 <= (size_t)tp->fused_dyn_max;
+}
+
+// The fused view step's item table for the split count in use, built on first use (it allocates:
+// outside any capture) and kept with the work set.
+int tc_items(const Psf* psf, TcSolverState* t) {
+  if (t->items.count(t->splits)) return MLF_OK;
+  std::vector<int> tiles;
+  for (int p = 0; p < t->P; ++p) tiles.push_back((t->LL[p] + BM - 1) / BM);
+  const std::vector<ItemCost> costs =
+      item_costs(psf->N * psf->N, psf->tc->KB, psf->tc->NB, tiles, t->z0, t->nz, t->splits);
+  const int grid = std::min((int)costs.size(), t->nsm);
+  std::vector<std::vector<int>> lists(grid);
+  assign_items(costs, grid, &lists);
+  size_t rounds = 0;
+  for (const auto& l : lists) rounds = std::max(rounds, l.size());
+  std::vector<int> tab(rounds * grid, -1);
+  for (int c = 0; c < grid; ++c)
+    for (size_t k = 0; k < lists[c].size(); ++k) tab[k * grid + c] = lists[c][k];
+  TcSolverState::Items& e = t->items[t->splits];
+  e.n = (int)tab.size();
+  e.grid = grid;
+  e.identity = true;
+  for (size_t k = 0; k < tab.size(); ++k) e.identity = e.identity && tab[k] == (int)k;
+  int rc = e.tab.alloc(tab.size() * sizeof(int), "tc item table");
+  if (rc == MLF_OK && cudaMemcpy(e.tab.p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+    rc = fail(MLF_ERR_CUDA, "tc item table upload");
+  if (rc != MLF_OK) t->items.erase(t->splits);
+  return rc;
 }
 
 int tc_bwdfwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, int view_next, const float* wrow,
@@ -2081,12 +2207,12 @@ int tc_bwdfwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, 
   a.MP = t->MP;
   a.NB = tp->NB;
   a.splits = t->splits;
-  a.ks_per_split = t->ks_per_split;
   a.KS = t->KSF;
   a.frow0 = view_next * tp->NB;
-  a.ntiles = tp->CHP / BWD_BN;
-  const int nitems = (t->MP / BM) * t->splits;
-  const int grid = std::min(nitems, t->nsm);
+  const auto it = t->items.find(t->splits);
+  if (it == t->items.end()) return fail(MLF_ERR_INVALID, "fused view step: item table not prepared");
+  a.items = it->second.identity ? nullptr : it->second.tab.as<int>();
+  const int nitems = it->second.n, grid = it->second.grid;
   // (X buffers, ring stages): (2, 2), or (1, 3) where two X buffers do not fit or the
   // environment sets MLF_FUSED_XB=1 (slower on the 1005 x 1005 x 51 workload: 0.218 vs
   // 0.189 ms per view, the single X buffer serialises the tiles)
@@ -2195,19 +2321,18 @@ void tc_apply_tune(TcSolverState* t, int precision) {
   const TcSolverState::Tune& g = t->tune[precision];
   if (g.done) {
     t->splits = g.splits;
-    t->ks_per_split = g.ksp;
     t->fwd_stages = g.fwd_stages;
     t->xbufs = g.xbufs;
   } else {
     t->splits = t->splits_def;
-    t->ks_per_split = t->ksp_def;
     t->fwd_stages = 0;
     t->xbufs = 0;
   }
 }
 
 // Autotuner: time the candidate launch configurations on the first view step of the work
-// set (forward GEMM: split-K count in {s/2, s, 2s} x ring depth in {2, 3, 4}; back
+// set (split-K count in {s/2, s, 2s}, on the fused view step with the sum over its splits where
+// that runs and on the forward GEMM elsewhere; the forward GEMM's ring depth in {2, 3, 4}; back
 // projection: one or two X buffers per half) and keep the fastest.  X is saved before and
 // restored after, so the solve is unaffected.  Runs once per work set and precision, before
 // the iteration is captured; MLF_TUNE=0 keeps the heuristics.
@@ -2216,7 +2341,6 @@ int tc_autotune(const Psf* psf, TcSolverState* t, int precision, cudaStream_t st
   if (g.done) return MLF_OK;
   g.done = 1;
   g.splits = t->splits_def;
-  g.ksp = t->ksp_def;
   const char* env = std::getenv("MLF_TUNE");
   if ((env && std::strcmp(env, "0") == 0) || t->views.empty()) return MLF_OK;
   DevBuf xsave;
@@ -2237,28 +2361,58 @@ int tc_autotune(const Psf* psf, TcSolverState* t, int precision, cudaStream_t st
   };
   const int v0 = t->views[0];
   const float* w0 = t->wtab_dev.as<float>();
+  const int V = (int)t->views.size();
+  const bool fused = V > 1 && tc_fused_ok(psf, t, precision);
+  if (fused) {  // the view step needs a ratio image
+    MLF_TRY(tc_fwd_launch(psf, t, precision, v0, st, w0));
+    MLF_TRY(tc_col2im(psf, t, v0, true, nullptr, st, precision, 0));
+    MLF_TRY(tc_im2col_ratio(psf, t, precision, st, 0));
+  }
   float best = 1e30f;
-  for (int s : {std::max(1, t->splits_def / 2), t->splits_def, t->splits_max}) {
-    const int ksp = (((t->KSF + s - 1) / s) + 1) & ~1;
-    const int sp = (t->KSF + ksp - 1) / ksp;
-    if (sp > t->splits_max) continue;
+  int last = 0;
+  for (int sp : {std::max(1, t->splits_def / 2), t->splits_def, t->splits_max}) {
+    if (sp == last) continue;
+    last = sp;
+    t->splits = sp;
+    float ms = 0.f;
+    if (fused) {
+      MLF_TRY(tc_items(psf, t));
+      MLF_TRY(timed([&]() -> int {
+        MLF_TRY(tc_bwdfwd_launch(psf, t, precision, v0, t->views[1], w0, w0 + t->P, st));
+        return tc_col2im(psf, t, t->views[1], false, nullptr, st, precision, 0);
+      }, &ms));
+      if (ms < best) {
+        best = ms;
+        g.splits = sp;
+      }
+      continue;
+    }
     for (int stg = 2; stg <= FWD_MAX_STAGES; ++stg) {
-      t->splits = sp;
-      t->ks_per_split = ksp;
+      t->fwd_stages = stg;
+      MLF_TRY(timed([&] { return tc_fwd_launch(psf, t, precision, v0, st, w0); }, &ms));
+      if (ms < best) {
+        best = ms;
+        g.splits = sp;
+        g.fwd_stages = stg;
+      }
+    }
+  }
+  if (fused) {
+    t->splits = g.splits;
+    best = 1e30f;
+    for (int stg = 2; stg <= FWD_MAX_STAGES; ++stg) {
       t->fwd_stages = stg;
       float ms = 0.f;
       MLF_TRY(timed([&] { return tc_fwd_launch(psf, t, precision, v0, st, w0); }, &ms));
       if (ms < best) {
         best = ms;
-        g.splits = sp;
-        g.ksp = ksp;
         g.fwd_stages = stg;
       }
     }
+    MLF_CUDA(cudaMemcpyAsync(t->X.p, xsave.p, t->X.bytes, cudaMemcpyDeviceToDevice, st));
   }
   // the back projection needs the ratio image of view 0 under the chosen forward
   t->splits = g.splits;
-  t->ks_per_split = g.ksp;
   t->fwd_stages = g.fwd_stages;
   MLF_TRY(tc_fwd_launch(psf, t, precision, v0, st, w0));
   MLF_TRY(tc_col2im(psf, t, v0, true, nullptr, st, precision, 0));
@@ -2342,6 +2496,7 @@ int tc_run(TcSolverState* t, const std::vector<Solver*>& members, const std::vec
   if (max_iter > 0) {
     MLF_TRY(tc_autotune(psf, t, precision, st));  // first solve at this precision only
     tc_apply_tune(t, precision);
+    if (tc_fused_ok(psf, t, precision)) MLF_TRY(tc_items(psf, t));
     if (monitor) MLF_CUDA(cudaMemcpyAsync(t->Xprev.p, t->X.p, t->X.bytes, cudaMemcpyDeviceToDevice, st));
     TcSolverState::Iteration& g = t->iter[precision][timer->timing ? 1 : 0];
     if (!g.exec) {
