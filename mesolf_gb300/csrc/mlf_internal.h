@@ -172,7 +172,9 @@ struct Solver {
   int Pa = 0;          // row pitch (floats) of a phase-major plane (FP32 kernels)
   int64_t plane = 0;   // floats per plane (Lj * Pa)
   int64_t nch = 0;
-  // view-kernel geometry
+  // view-kernel geometry (tileY x tileX: the kernel's tile)
+  bool small = false;  // the view kernel's small tile
+  int tileY = 0, tileX = 0;
   int tilesA = 0, tilesB = 0, tps = 0, slots = 0, tstride = 0, threads = 0, grid = 0;
   int RP = 0, RProws = 0, XP = 0, XProws = 0, maxc = 0;
   size_t smem = 0;
@@ -181,7 +183,7 @@ struct Solver {
   DevBuf Xtmp;       // float [nch][plane]      scratch volume (back-projection output, filter)
   DevBuf lfs;        // float [N*N][Lj*Li]      sub-aperture images
   DevBuf rpad;       // float [RProws][RP]      halo-padded ratio image
-  DevBuf part;       // float [grid][slots][tilesB*VW_TY][tilesA*VW_TX] per-slot forward partials
+  DevBuf part;       // float [grid][slots][tilesB*tileY][tilesA*tileX] per-slot forward partials
   DevBuf hx;         // float [Lj*Li]           last forward projection
   DevBuf cls;        // int tables: clsA[3][Li], clsB[3][Lj], rngA[3][maxc][2], rngB[3][maxc][2]
   DevBuf red;        // double scratch for reductions
@@ -308,7 +310,7 @@ struct ViewArgs {
   const float* rpad;   // halo-padded ratio image
   const float* wb;     // backward taps of the current view [nch][T*T]
   const float* wf;     // forward taps of the view being projected [nch][T*T]
-  float* part;         // [gridDim.x * slots][tilesB*VW_TY][tilesA*VW_TX] forward partials
+  float* part;         // [gridDim.x * slots][tilesB*TY][tilesA*TX] forward partials (TY x TX: the tile)
   const int* clsA;     // [3][Li]
   const int* clsB;     // [3][Lj]
   const int* rngA;     // [3][maxc][2]
@@ -321,6 +323,7 @@ struct ViewArgs {
   int64_t plane, nch;
   int tilesA, tilesB, tps, slots, tstride;  // tstride: threads per slot (>= tps)
   int RP, RProws, XP, XProws, maxc, slot_floats;
+  int small;           // the small tile
   CancelRef cancel;    // all null: not cancellable
 };
 enum ViewMode { MODE_FWD = 0, MODE_STEP = 1, MODE_BWDC = 2 };
@@ -340,6 +343,9 @@ constexpr int view_nw(int T) { return (4 + T - 1 + view_offmax((T - 1) / 2) + 3)
 // above (8 b x 4 a) is the allocation-free forward projection's.
 constexpr int VW_TY = 4;
 constexpr int VW_TX = 8;
+// The small tile, for patches whose channels give the 4 x 8 tile too few threads (solver_init).
+constexpr int VWS_TY = 2;
+constexpr int VWS_TX = 4;
 // threads per view-kernel CTA at most (two slots of up to 160 tiles)
 constexpr int kViewMaxThreads = 320;
 // Whether a CTA adds its slots' forward partials itself (the comment at the sum in k_view).
@@ -355,9 +361,10 @@ __host__ __device__ inline int view_pcol(int c, int pitch) {
 }
 // Smallest pitch >= need (floats) that is 4 mod 8.
 __host__ __device__ constexpr int view_plane_pitch(int need) { return ((need + 3) & ~7) + 4; }
-constexpr int view_nw8(int T) { return (VW_TX + T - 1 + view_offmax((T - 1) / 2) + 3) / 4; }
-int prepare_view_kernels(int T, size_t smem);
-int occupancy_view_kernel(int T, int threads, size_t smem, int* blocks);
+// float4 loads per window row of a tile of TX columns
+constexpr int view_nw(int T, int TX) { return (TX + T - 1 + view_offmax((T - 1) / 2) + 3) / 4; }
+int prepare_view_kernels(int T, bool small);
+int occupancy_view_kernel(int T, bool small, int threads, size_t smem, int* blocks);
 int launch_view_kernel(int T, int mode, const ViewArgs& a, int grid, int threads, size_t smem,
                        cudaStream_t st);
 bool view_taps_supported(int T);

@@ -238,9 +238,14 @@ k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int H
   sh[grp][lane] = s;
   __syncthreads();
   if (grp != 0 || i >= LL) return;
-  float hx = 0.f;
+  float t[kReduceGroups];  // pairwise: a short chain, and a rounding error that does not grow with it
 #pragma unroll
-  for (int g = 0; g < kReduceGroups; ++g) hx += sh[g][lane];
+  for (int g = 0; g < kReduceGroups; ++g) t[g] = sh[g][lane];
+#pragma unroll
+  for (int h = kReduceGroups / 2; h > 0; h /= 2)
+#pragma unroll
+    for (int g = 0; g < h; ++g) t[g] += t[g + h];
+  const float hx = t[0];
   if (hx_out) hx_out[i] = hx;
   if (rpad) {
     float r = lfsub[i] / hx;
@@ -282,6 +287,7 @@ ViewArgs view_args(Solver* s) {
   a.N = s->N; a.Z = s->Z; a.Li = s->Li; a.Lj = s->Lj; a.Pa = s->Pa; a.q = s->q;
   a.plane = s->plane; a.nch = s->nch;
   a.tilesA = s->tilesA; a.tilesB = s->tilesB; a.tps = s->tps; a.slots = s->slots; a.tstride = s->tstride;
+  a.small = s->small ? 1 : 0;
   a.RP = s->RP; a.RProws = s->RProws; a.XP = s->XP; a.XProws = s->XProws; a.maxc = s->maxc;
   a.cancel = CancelRef{nullptr, nullptr, nullptr};  // solves set it (enqueue_iteration)
   a.slot_floats = round_up(s->XProws * s->XP + 4 * s->T * view_tap_pitch(s->T) + s->maxc * s->maxc + s->T * s->maxc, 4);
@@ -366,10 +372,10 @@ int run_view(Solver* s, int mode, int view_cur, int view_next, float w, bool do_
 int run_reduce(Solver* s, int view, float* hx_out, bool ratio, cudaStream_t st) {
   const int LL = s->Li * s->Lj;
   const float* lfsub = s->lfs.as<float>() + (int64_t)view * LL;
-  const int HP = s->tilesA * VW_TX;
+  const int HP = s->tilesA * s->tileX;
   const int group = view_sums_slots(s->slots) ? s->slots : 1;  // planes that the view kernel has added
   k_reduce_ratio<<<ceil_div(LL, 32), 32 * kReduceGroups, 0, st>>>(
-      s->part.as<float>(), s->grid * s->slots / group, s->Li, s->Lj, HP, (int64_t)group * s->tilesB * VW_TY * HP, lfsub, hx_out,
+      s->part.as<float>(), s->grid * s->slots / group, s->Li, s->Lj, HP, (int64_t)group * s->tilesB * s->tileY * HP, lfsub, hx_out,
       ratio ? s->rpad.as<float>() : nullptr, s->RP, s->q + 1);
   MLF_LAUNCHED();
   return MLF_OK;
@@ -603,18 +609,28 @@ int solver_init(Solver* s) {
   if (s->nch * (int64_t)s->T * s->T >= (int64_t)INT32_MAX)
     return fail(MLF_ERR_UNSUPPORTED, "too many depth planes for the view kernel's 32-bit channel indices");
   if (s->lite) return MLF_OK;  // batch member: geometry now, filter plan and scratch on first solve
-  s->tilesA = ceil_div(s->Li, VW_TX);
-  s->tilesB = ceil_div(s->Lj, VW_TY);
+  // Tile: 2 x 4 outputs per thread where the 4 x 8 tile would leave the chip with a warp or two
+  // per scheduler, so that a view step is a chain of latencies and not the instructions of 32
+  // outputs in a row.  The line lies where the larger tile's fewer shared loads per FMA begin to
+  // count (threads of the 4 x 8 tile, 2 iterations): 28 K (11 x 11 x 21, T 3) 4.7 -> 3.5 ms,
+  // 55 K (11 x 12 x 41, T 15) 33.3 -> 21.4, 94 K (15 x 40 x 21, T 7) 10.4 -> 9.7, 108 K (30 x 30 x
+  // 15, T 9) 12.4 -> 11.5, but 134 K (24 x 24 x 33, T 7) 12.7 -> 13.4.
+  s->small = ceil_div(s->Li, VWS_TX) * ceil_div(s->Lj, VWS_TY) <= 256 &&
+             s->nch * ceil_div(s->Li, VW_TX) * ceil_div(s->Lj, VW_TY) <= 120000;
+  s->tileY = s->small ? VWS_TY : VW_TY;
+  s->tileX = s->small ? VWS_TX : VW_TX;
+  s->tilesA = ceil_div(s->Li, s->tileX);
+  s->tilesB = ceil_div(s->Lj, s->tileY);
   s->tps = s->tilesA * s->tilesB;
   if (s->tps > 256)
     return fail(MLF_ERR_UNSUPPORTED, "patch of " + std::to_string(s->Li) + " x " +
                                          std::to_string(s->Lj) +
                                          " lenslets exceeds the 128 x 64 per-solve limit; tile the field of view");
-  const int NW = view_nw8(s->T);
-  s->RP = view_plane_pitch(VW_TX * (s->tilesA - 1) + 4 * NW);
-  s->RProws = s->tilesB * VW_TY + s->T + 1;
+  const int NW = view_nw(s->T, s->tileX);
+  s->RP = view_plane_pitch(s->tileX * (s->tilesA - 1) + 4 * NW);
+  s->RProws = s->tilesB * s->tileY + s->T + 1;
   s->XP = s->RP;
-  s->XProws = s->tilesB * VW_TY + s->T - 1;
+  s->XProws = s->tilesB * s->tileY + s->T - 1;
 
   std::vector<int> clsA, clsB;
   std::vector<std::pair<int, int>> rngA[3], rngB[3];
@@ -644,7 +660,7 @@ int solver_init(Solver* s) {
   MLF_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
   MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
   // Channel slots per CTA (they share the staged ratio image).  Small patches: as many as
-  // the shared memory holds, up to 192 threads.  Patches of 128..160 tiles: two slots when
+  // the shared memory holds, up to 192 threads, while every SM has two CTAs.  Patches of 128..160 tiles: two slots when
   // two such CTAs fit an SM's shared memory (20 warps per SM instead of 15); larger: one.
   const int64_t R_floats = (int64_t)s->RProws * s->RP;
   const int64_t fit = ((int64_t)dev_smem / (int64_t)sizeof(float) - R_floats) / slot_floats;
@@ -652,7 +668,8 @@ int solver_init(Solver* s) {
   MLF_CUDA(cudaDeviceGetAttribute(&sm_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device));
   const int64_t two_slot_bytes = (int64_t)sizeof(float) * (R_floats + 2 * (int64_t)slot_floats);
   if (s->tps < 128)
-    s->slots = std::max(1, std::min({32, 192 / s->tps, (int)std::max<int64_t>(1, fit)}));
+    s->slots = std::max(1, std::min({32, 192 / s->tps, (int)std::max<int64_t>(1, fit),
+                                     (int)std::min<int64_t>(32, (s->nch + 2 * nsm - 1) / (2 * nsm))}));
   else
     s->slots = (2 * s->tps <= kViewMaxThreads && 2 * (two_slot_bytes + 1024) <= sm_per_sm) ? 2 : 1;
   // several slots: each starts on a warp boundary when that costs no extra warp
@@ -661,9 +678,9 @@ int solver_init(Solver* s) {
   s->threads = round_up(s->slots * s->tstride, 32);
   s->smem = sizeof(float) * ((size_t)s->RProws * s->RP + (size_t)s->slots * slot_floats);
   if ((int)s->smem > dev_smem) return fail(MLF_ERR_UNSUPPORTED, "view kernel shared memory exceeds the device limit");
-  MLF_TRY(prepare_view_kernels(s->T, s->smem));
+  MLF_TRY(prepare_view_kernels(s->T, s->small));
   int per_sm = 1;
-  MLF_TRY(occupancy_view_kernel(s->T, s->threads, s->smem, &per_sm));
+  MLF_TRY(occupancy_view_kernel(s->T, s->small, s->threads, s->smem, &per_sm));
   per_sm = std::max(1, per_sm);
   const int64_t max_blocks = (s->nch + s->slots - 1) / s->slots;
   s->grid = (int)std::min<int64_t>(max_blocks, (int64_t)nsm * per_sm);
@@ -674,7 +691,7 @@ int solver_init(Solver* s) {
   MLF_TRY(s->Xtmp.alloc(vol * sizeof(float), "scratch volume"));
   MLF_TRY(s->lfs.alloc((size_t)s->N * s->N * LL * sizeof(float), "sub-aperture images"));
   MLF_TRY(s->rpad.alloc((size_t)s->RProws * s->RP * sizeof(float), "ratio image"));
-  MLF_TRY(s->part.alloc((size_t)s->grid * s->slots * (s->tilesB * VW_TY) * (s->tilesA * VW_TX) * sizeof(float),
+  MLF_TRY(s->part.alloc((size_t)s->grid * s->slots * (s->tilesB * s->tileY) * (s->tilesA * s->tileX) * sizeof(float),
                         "forward partials"));
   MLF_TRY(s->hx.alloc(LL * sizeof(float), "forward projection"));
   MLF_TRY(s->red.alloc(4096 * sizeof(double), "reduction scratch"));
@@ -911,8 +928,8 @@ int sample_filter(Solver* s, float* d_vol, cudaStream_t st) {
 
 // ---------------------------------------------------------------- dispatch per T
 #define MLF_DECL_T(T)                                                                     \
-  int prepare_view_T##T(size_t smem);                                                    \
-  int occupancy_view_T##T(int threads, size_t smem, int* blocks);                        \
+  int prepare_view_T##T(bool small);                                                     \
+  int occupancy_view_T##T(bool small, int threads, size_t smem, int* blocks);            \
   int launch_view_T##T(int mode, const ViewArgs& a, int grid, int threads, size_t smem, \
                        cudaStream_t st);
 MLF_DECL_T(3) MLF_DECL_T(5) MLF_DECL_T(7) MLF_DECL_T(9) MLF_DECL_T(11) MLF_DECL_T(13) MLF_DECL_T(15) MLF_DECL_T(17)
@@ -931,13 +948,13 @@ MLF_DECL_T(3) MLF_DECL_T(5) MLF_DECL_T(7) MLF_DECL_T(9) MLF_DECL_T(11) MLF_DECL_
     default: return fail(MLF_ERR_UNSUPPORTED, "unsupported tap count"); \
   }
 
-int prepare_view_kernels(int T, size_t smem) {
-#define E(t) prepare_view_T##t(smem)
+int prepare_view_kernels(int T, bool small) {
+#define E(t) prepare_view_T##t(small)
   MLF_CASES(E)
 #undef E
 }
-int occupancy_view_kernel(int T, int threads, size_t smem, int* blocks) {
-#define E(t) occupancy_view_T##t(threads, smem, blocks)
+int occupancy_view_kernel(int T, bool small, int threads, size_t smem, int* blocks) {
+#define E(t) occupancy_view_T##t(small, threads, smem, blocks)
   MLF_CASES(E)
 #undef E
 }

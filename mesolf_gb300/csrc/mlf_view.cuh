@@ -87,25 +87,25 @@ __device__ __forceinline__ void conv_tile(const float* __restrict__ in, int pitc
 }
 
 // acc[ty][tx] += sum_{dy<T, dx<T} in[(ty+dy)*pitch + col(OFF + tx + dx)] * w[dy*WP+dx]
-// for the 4 x 8 tile of the view kernel, on a plane whose columns are swizzled in 16-byte
+// for a TY x TX tile of the view kernel, on a plane whose columns are swizzled in 16-byte
 // chunks: chunk k of this thread's window (columns a0 + 4k .. a0 + 4k + 3) starts at column
-// view_pcol(a0 + 4k, pitch) of a row.  Walks the VW_TY + T - 1 input rows once: row r is loaded
+// view_pcol(a0 + 4k, pitch) of a row.  Walks the TY + T - 1 input rows once: row r is loaded
 // into registers once and serves every output row ty with a tap row dy = r - ty (tap rows
 // come from shared memory as broadcast 16-byte loads), so the input window is read once
 // per tile instead of once per tap row.  Per output the products are added in the order
 // dy, then dx -- the order of conv_tile -- so the results are the same bit for bit.
 // `in` 16-byte aligned, a0 and pitch multiples of 4, WP a multiple of 4.
-template <int T, int OFF, int WP>
+template <int T, int OFF, int WP, int TY, int TX>
 __device__ __forceinline__ void conv_rows(const float* __restrict__ in, int pitch, int a0,
-                                          const float* __restrict__ w, float (&acc)[VW_TY][VW_TX]) {
-  constexpr int NW = view_nw8(T);
-  static_assert(OFF + VW_TX + T - 1 <= 4 * NW, "window too short");
+                                          const float* __restrict__ w, float (&acc)[TY][TX]) {
+  constexpr int NW = view_nw(T, TX);
+  static_assert(OFF + TX + T - 1 <= 4 * NW, "window too short");
   static_assert(WP % 4 == 0, "tap rows must be 16-byte aligned");
   int off[NW];
 #pragma unroll
   for (int k = 0; k < NW; ++k) off[k] = view_pcol(a0 + 4 * k, pitch);
 #pragma unroll 1
-  for (int r = 0; r < VW_TY + T - 1; ++r) {
+  for (int r = 0; r < TY + T - 1; ++r) {
     float win[4 * NW];
     const float* row = in + r * pitch;
 #pragma unroll
@@ -117,7 +117,7 @@ __device__ __forceinline__ void conv_rows(const float* __restrict__ in, int pitc
       win[4 * k + 3] = t4.w;
     }
 #pragma unroll
-    for (int ty = 0; ty < VW_TY; ++ty) {
+    for (int ty = 0; ty < TY; ++ty) {
       const int dy = r - ty;
       if (dy < 0 || dy >= T) continue;
       float wr[T];
@@ -133,7 +133,7 @@ __device__ __forceinline__ void conv_rows(const float* __restrict__ in, int pitc
 #pragma unroll
       for (int dx = 0; dx < T; ++dx)
 #pragma unroll
-        for (int tx = 0; tx < VW_TX; ++tx) acc[ty][tx] = fmaf(win[OFF + tx + dx], wr[dx], acc[ty][tx]);
+        for (int tx = 0; tx < TX; ++tx) acc[ty][tx] = fmaf(win[OFF + tx + dx], wr[dx], acc[ty][tx]);
     }
   }
 }
@@ -199,8 +199,10 @@ __device__ __forceinline__ void view_d_table(const ViewArgs& A, int ch, int lt, 
 }
 
 // At most kViewMaxThreads threads and two CTAs per SM: 96 registers per thread.
-template <int T, int MODE>
+template <int T, int MODE, int TY, int TX>
 __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
+  static_assert(TX % 4 == 0, "tile rows are whole 16-byte chunks");
+  constexpr int NC = TX / 4;             // 16-byte chunks of a tile row
   extern __shared__ __align__(16) float sm[];
   constexpr int TT = T * T;
   constexpr int TW = view_tap_pitch(T);  // tap-row pitch in shared memory
@@ -228,17 +230,15 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     ta = lt % A.tilesA;
     tb = lt / A.tilesA;
   }
-  const int a0 = ta * VW_TX, b0 = tb * VW_TY;
-  // swizzled columns of this tile's two X chunks in the forward-input plane
-  const int xc0 = view_pcol(a0 + QP, A.XP), xc1 = view_pcol(a0 + QP + 4, A.XP);
+  const int a0 = ta * TX, b0 = tb * TY;
+  int xc[NC];  // swizzled columns of this tile's X chunks in the forward-input plane
+#pragma unroll
+  for (int k = 0; k < NC; ++k) xc[k] = view_pcol(a0 + QP + 4 * k, A.XP);
 
-  // ---- a cancelled solve: the rest of its view steps return at once (CTA-uniform)
-  {
-    __shared__ int s_stop;
-    if (tid == 0) s_stop = cancel_entry(A.cancel);
-    __syncthreads();
-    if (s_stop) return;
-  }
+  // ---- a cancelled solve: the rest of its view steps return at once (CTA-uniform, at the first
+  // barrier; until then nothing but shared memory is written)
+  __shared__ int s_stop;
+  if (tid == 0) s_stop = cancel_entry(A.cancel);
 
   // ---- shared memory carve-up
   float* rs = sm;                                              // [RProws][RP] (BWD only)
@@ -248,10 +248,15 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   float* dtab = taps + 4 * TTW;                                // [maxc][maxc]
   float* rowp = dtab + A.maxc * A.maxc;                        // [T][maxc]
 
-  // ---- zero the slots (halos must be zero), stage R
+  // ---- zero the forward-input planes (halos must be zero), stage R
   {
-    const int total = A.slots * A.slot_floats;
-    for (int i = tid; i < total; i += blockDim.x) slot_base[i] = 0.f;
+    if (XIN) {
+      const int n4 = A.XProws * A.XP / 4, total = A.slots * n4;
+      for (int i = tid; i < total; i += blockDim.x) {
+        const int sl = i / n4;
+        reinterpret_cast<float4*>(slot_base + sl * A.slot_floats)[i - sl * n4] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
     if (BWD) {
       const int nr = A.RProws * A.RP;
       const float4* src = reinterpret_cast<const float4*>(A.rpad);
@@ -266,11 +271,11 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   const int nch = (int)A.nch;
   const int step = (int)gridDim.x * A.slots;
   const int first = (int)blockIdx.x * A.slots + slot;
-  // this thread's tile in its slot's forward partial plane [tilesB*VW_TY][tilesA*VW_TX]
+  // this thread's tile in its slot's forward partial plane [tilesB*TY][tilesA*TX]
   // (tile rows 32-byte aligned); recomputed where used rather than held across the loop
   auto hx_tile = [&]() {
-    const int HP = A.tilesA * VW_TX;
-    return A.part + ((int64_t)blockIdx.x * A.slots + (slot_ok ? slot : 0)) * ((int64_t)A.tilesB * VW_TY * HP) +
+    const int HP = A.tilesA * TX;
+    return A.part + ((int64_t)blockIdx.x * A.slots + (slot_ok ? slot : 0)) * ((int64_t)A.tilesB * TY * HP) +
            (int64_t)b0 * HP + a0;
   };
   bool hx_written = false;
@@ -286,6 +291,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     if (DT) view_d_rows<T>(A, first, lt, rowp);
   }
   __syncthreads();
+  if (s_stop) return;
   if (DT && slot_ok && first < nch) view_d_table<T>(A, first, lt, rowp, dtab);
   __syncthreads();
 
@@ -303,16 +309,17 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     const float* wfs = wbs + TTW;
 
     // ---- X tile -> forward-input plane (interior at rows +Q, cols +QP), asynchronously.
-    // A plane row has Pa (a multiple of 4) floats: the second 16-byte half of the last tile
-    // may lie past it and is then not copied (its shared-memory cells stay zero).
+    // A plane row has Pa (a multiple of 4) floats: a 16-byte chunk of the last tile may
+    // lie past it and is then not copied (its shared-memory cells stay zero).
     if (XIN && active) {
       const float* Xch = A.X + ch * A.plane;
 #pragma unroll
-      for (int y = 0; y < VW_TY; ++y) {
+      for (int y = 0; y < TY; ++y) {
         const int b = b0 + y;
         if (b >= A.Lj) continue;
-        cp_async16(xin + (b + Q) * A.XP + xc0, Xch + (int64_t)b * A.Pa + a0);
-        if (a0 + 4 < A.Pa) cp_async16(xin + (b + Q) * A.XP + xc1, Xch + (int64_t)b * A.Pa + a0 + 4);
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+          if (a0 + 4 * k < A.Pa) cp_async16(xin + (b + Q) * A.XP + xc[k], Xch + (int64_t)b * A.Pa + a0 + 4 * k);
       }
     }
 
@@ -324,36 +331,36 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
       if (active && ph == 0 && !BWD) {
         cp_async_wait_all();  // forward only: this thread's X tile has landed in xin
       } else if (active) {
-        float acc[VW_TY][VW_TX];
+        float acc[TY][TX];
 #pragma unroll
-        for (int y = 0; y < VW_TY; ++y)
+        for (int y = 0; y < TY; ++y)
 #pragma unroll
-          for (int x = 0; x < VW_TX; ++x) acc[y][x] = 0.f;
+          for (int x = 0; x < TX; ++x) acc[y][x] = 0.f;
         if (ph == 1 && hx_written) {  // this tile's forward partials into L1 for the add below
           const float* hxp = hx_tile();
 #pragma unroll
-          for (int y = 0; y < VW_TY; ++y)
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(hxp + y * A.tilesA * VW_TX));
+          for (int y = 0; y < TY; ++y)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(hxp + y * A.tilesA * TX));
         }
         const float* in = ph == 0 ? rs + (b0 + sb + 1) * A.RP : xin + b0 * A.XP;
         const int pitch = ph == 0 ? A.RP : A.XP;
         const float* wsel = ph == 0 ? wbs : wfs;
         switch (ph == 0 ? sa + 1 : QP - Q) {
-          case 0: conv_rows<T, 0, TW>(in, pitch, a0, wsel, acc); break;
-          case 1: conv_rows<T, 1, TW>(in, pitch, a0, wsel, acc); break;
-          case 2: conv_rows<T, 2, TW>(in, pitch, a0, wsel, acc); break;
+          case 0: conv_rows<T, 0, TW, TY, TX>(in, pitch, a0, wsel, acc); break;
+          case 1: conv_rows<T, 1, TW, TY, TX>(in, pitch, a0, wsel, acc); break;
+          case 2: conv_rows<T, 2, TW, TY, TX>(in, pitch, a0, wsel, acc); break;
           default:
-            if constexpr (QP - Q == 3) conv_rows<T, 3, TW>(in, pitch, a0, wsel, acc);
+            if constexpr (QP - Q == 3) conv_rows<T, 3, TW, TY, TX>(in, pitch, a0, wsel, acc);
             break;
         }
         if (ph == 0) {
           if (MODE == MODE_BWDC) {
 #pragma unroll
-            for (int y = 0; y < VW_TY; ++y) {
+            for (int y = 0; y < TY; ++y) {
               const int b = b0 + y;
               if (b >= A.Lj) continue;
 #pragma unroll
-              for (int x = 0; x < VW_TX; ++x)
+              for (int x = 0; x < TX; ++x)
                 if (a0 + x < A.Li) A.Cout[(int64_t)ch * A.plane + (int64_t)b * A.Pa + a0 + x] = acc[y][x];
             }
           } else {
@@ -362,17 +369,22 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
             const int* cB = A.clsB + (sb + 1) * A.Lj;
             float* Xch = A.X + ch * A.plane;
 #pragma unroll
-            for (int y = 0; y < VW_TY; ++y) {
+            for (int y = 0; y < TY; ++y) {
               const int b = b0 + y;
               if (b >= A.Lj) continue;
               const int cb = __ldg(cB + b);
               float* xrow = xin + (b + Q) * A.XP;
-              const float4 x0 = *reinterpret_cast<const float4*>(xrow + xc0);
-              const float4 x1 = *reinterpret_cast<const float4*>(xrow + xc1);
-              const float xo8[VW_TX] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-              float xn8[VW_TX];
+              float xo8[TX], xn8[TX];
 #pragma unroll
-              for (int x = 0; x < VW_TX; ++x) {
+              for (int k = 0; k < NC; ++k) {
+                const float4 v = *reinterpret_cast<const float4*>(xrow + xc[k]);
+                xo8[4 * k] = v.x;
+                xo8[4 * k + 1] = v.y;
+                xo8[4 * k + 2] = v.z;
+                xo8[4 * k + 3] = v.w;
+              }
+#pragma unroll
+              for (int x = 0; x < TX; ++x) {
                 const int a = a0 + x;
                 const float xo = xo8[x];
                 xn8[x] = xo;  // columns past the patch keep their (zero) value
@@ -385,33 +397,44 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
                 if (xn < 0.f) xn = 0.f;                      // :137
                 xn8[x] = xn;
               }
-              const float4 n0 = make_float4(xn8[0], xn8[1], xn8[2], xn8[3]);
-              const float4 n1 = make_float4(xn8[4], xn8[5], xn8[6], xn8[7]);
-              *reinterpret_cast<float4*>(xrow + xc0) = n0;
-              *reinterpret_cast<float4*>(xrow + xc1) = n1;
               // the plane row has Pa (a multiple of 4) floats: its padding columns get back
-              // their own values; a second half past the row is not written
+              // their own values; a chunk past the row is not written
               float4* g = reinterpret_cast<float4*>(Xch + (int64_t)b * A.Pa + a0);
-              g[0] = n0;
-              if (a0 + 4 < A.Pa) g[1] = n1;
+#pragma unroll
+              for (int k = 0; k < NC; ++k)
+                *reinterpret_cast<float4*>(xrow + xc[k]) =
+                    make_float4(xn8[4 * k], xn8[4 * k + 1], xn8[4 * k + 2], xn8[4 * k + 3]);
+              g[0] = make_float4(xn8[0], xn8[1], xn8[2], xn8[3]);
+#pragma unroll
+              for (int k = 1; k < NC; ++k)
+                if (a0 + 4 * k < A.Pa) g[k] = make_float4(xn8[4 * k], xn8[4 * k + 1], xn8[4 * k + 2], xn8[4 * k + 3]);
             }
           }
         } else {
-          // forward partials: plane += this channel's projection (tile rows are 32 bytes)
+          // forward partials: plane += this channel's projection (tile rows are 16-byte chunks)
           float* hxp = hx_tile();
-          const int HP = A.tilesA * VW_TX;
+          const int HP = A.tilesA * TX;
 #pragma unroll
-          for (int y = 0; y < VW_TY; ++y) {
+          for (int y = 0; y < TY; ++y) {
             float4* p4 = reinterpret_cast<float4*>(hxp + y * HP);
-            float4 lo = make_float4(acc[y][0], acc[y][1], acc[y][2], acc[y][3]);
-            float4 hi = make_float4(acc[y][4], acc[y][5], acc[y][6], acc[y][7]);
+            float4 v[NC];
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+              v[k] = make_float4(acc[y][4 * k], acc[y][4 * k + 1], acc[y][4 * k + 2], acc[y][4 * k + 3]);
             if (hx_written) {
-              const float4 o0 = p4[0], o1 = p4[1];
-              lo.x = o0.x + lo.x; lo.y = o0.y + lo.y; lo.z = o0.z + lo.z; lo.w = o0.w + lo.w;
-              hi.x = o1.x + hi.x; hi.y = o1.y + hi.y; hi.z = o1.z + hi.z; hi.w = o1.w + hi.w;
+              float4 o[NC];
+#pragma unroll
+              for (int k = 0; k < NC; ++k) o[k] = p4[k];
+#pragma unroll
+              for (int k = 0; k < NC; ++k) {
+                v[k].x = o[k].x + v[k].x;
+                v[k].y = o[k].y + v[k].y;
+                v[k].z = o[k].z + v[k].z;
+                v[k].w = o[k].w + v[k].w;
+              }
             }
-            p4[0] = lo;
-            p4[1] = hi;
+#pragma unroll
+            for (int k = 0; k < NC; ++k) p4[k] = v[k];
           }
           hx_written = true;
         }
@@ -445,7 +468,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   // has projected channels when blockIdx * slots + s < nch; the loop's last barrier orders its
   // writes before these reads.
   if ((MODE == MODE_FWD || (MODE == MODE_STEP && A.do_fwd)) && view_sums_slots(A.slots)) {
-    const int n4 = A.tilesB * VW_TY * A.tilesA * VW_TX / 4;
+    const int n4 = A.tilesB * TY * A.tilesA * TX / 4;
     const int used = min(A.slots, nch - (int)blockIdx.x * A.slots);
     float4* p0 = reinterpret_cast<float4*>(A.part) + (int64_t)blockIdx.x * A.slots * n4;
     for (int i = tid; i < n4; i += blockDim.x) {
@@ -463,28 +486,30 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   }
 }
 
+#define MLF_VIEW_TILE(T, MODE, SMALL) \
+  ((SMALL) ? (const void*)k_view<(T), MODE, VWS_TY, VWS_TX> : (const void*)k_view<(T), MODE, VW_TY, VW_TX>)
+
 #define MLF_INSTANTIATE_VIEW(T)                                                                  \
-  int prepare_view_T##T(size_t smem) {                                                          \
-    (void)smem;                                                                                 \
-    MLF_TRY(allow_max_dyn_smem((const void*)k_view<T, MODE_FWD>));                              \
-    MLF_TRY(allow_max_dyn_smem((const void*)k_view<T, MODE_STEP>));                             \
-    return allow_max_dyn_smem((const void*)k_view<T, MODE_BWDC>);                               \
+  int prepare_view_T##T(bool small) {                                                           \
+    MLF_TRY(allow_max_dyn_smem(MLF_VIEW_TILE(T, MODE_FWD, small)));                              \
+    MLF_TRY(allow_max_dyn_smem(MLF_VIEW_TILE(T, MODE_STEP, small)));                             \
+    return allow_max_dyn_smem(MLF_VIEW_TILE(T, MODE_BWDC, small));                               \
   }                                                                                             \
-  int occupancy_view_T##T(int threads, size_t smem, int* blocks) {                              \
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k_view<T, MODE_STEP>, \
-                                                                  threads, smem);               \
+  int occupancy_view_T##T(bool small, int threads, size_t smem, int* blocks) {                  \
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(                              \
+        blocks, MLF_VIEW_TILE(T, MODE_STEP, small), threads, smem);                              \
     if (e != cudaSuccess)                                                                       \
       return fail(MLF_ERR_CUDA, std::string("occupancy: ") + cudaGetErrorString(e));            \
     return MLF_OK;                                                                              \
   }                                                                                             \
   int launch_view_T##T(int mode, const ViewArgs& a, int grid, int threads, size_t smem,         \
                        cudaStream_t st) {                                                       \
-    switch (mode) {                                                                             \
-      case MODE_FWD: k_view<T, MODE_FWD><<<grid, threads, smem, st>>>(a); break;                \
-      case MODE_STEP: k_view<T, MODE_STEP><<<grid, threads, smem, st>>>(a); break;              \
-      default: k_view<T, MODE_BWDC><<<grid, threads, smem, st>>>(a); break;                     \
-    }                                                                                           \
-    cudaError_t e = cudaGetLastError();                                                         \
+    const void* f = mode == MODE_FWD ? MLF_VIEW_TILE(T, MODE_FWD, a.small)                      \
+                    : mode == MODE_STEP ? MLF_VIEW_TILE(T, MODE_STEP, a.small)                  \
+                                        : MLF_VIEW_TILE(T, MODE_BWDC, a.small);                 \
+    ViewArgs v = a;                                                                             \
+    void* args[] = {&v};                                                                        \
+    cudaError_t e = cudaLaunchKernel(f, dim3(grid), dim3(threads), args, smem, st);             \
     if (e != cudaSuccess)                                                                       \
       return fail(MLF_ERR_CUDA, std::string("view kernel launch: ") + cudaGetErrorString(e));   \
     return MLF_OK;                                                                              \
