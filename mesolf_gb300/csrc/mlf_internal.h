@@ -289,6 +289,16 @@ int launch_mex_pad_add(const float* src, int64_t W, int64_t H, int64_t Wp, int64
 int launch_mex_crop(const float* src, int64_t Wp, int64_t Hq, int64_t W, int64_t H, int64_t n, float* out,
                     cudaStream_t st);
 
+// Programmatic dependent launch: a kernel launched with launch_pdl may start before the kernel
+// before it in the stream has ended, and calls pdl_wait before it reads or overwrites anything that
+// kernel, or one before it, writes or reads.  Every launch_pdl kernel calls pdl_wait in all its
+// threads, so that the order of a chain of them is kept.
+cudaError_t launch_pdl(const void* f, int grid, int threads, void** args, size_t smem, cudaStream_t st);
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // Entry check of the cancellable kernels, by thread 0 (the caller broadcasts the result to
 // its CTA before any barrier): CTA 0 turns a host request into the stop words; every CTA
 // then returns when the device stop word is set.

@@ -216,6 +216,8 @@ k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int H
                const float* __restrict__ lfsub, float* __restrict__ hx_out,
                float* __restrict__ rpad, int RP, int off) {
   __shared__ float sh[kReduceGroups][32];
+  pdl_launch_dependents();
+  pdl_wait();
   const int LL = Li * Lj;
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
@@ -332,6 +334,20 @@ void build_classes(int L, int q, std::vector<int>& cls, std::vector<std::pair<in
 
 }  // namespace
 
+cudaError_t launch_pdl(const void* f, int grid, int threads, void** args, size_t smem, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, f, args);
+}
+
 int timing_mark(Solver* s, cudaStream_t st) {
   if (!s->timing) return MLF_OK;
   if (s->tev_used >= (int)s->tev.size()) {
@@ -374,10 +390,12 @@ int run_reduce(Solver* s, int view, float* hx_out, bool ratio, cudaStream_t st) 
   const float* lfsub = s->lfs.as<float>() + (int64_t)view * LL;
   const int HP = s->tilesA * s->tileX;
   const int group = view_sums_slots(s->slots) ? s->slots : 1;  // planes that the view kernel has added
-  k_reduce_ratio<<<ceil_div(LL, 32), 32 * kReduceGroups, 0, st>>>(
-      s->part.as<float>(), s->grid * s->slots / group, s->Li, s->Lj, HP, (int64_t)group * s->tilesB * s->tileY * HP, lfsub, hx_out,
-      ratio ? s->rpad.as<float>() : nullptr, s->RP, s->q + 1);
-  MLF_LAUNCHED();
+  const float* part = s->part.as<float>();
+  int nparts = s->grid * s->slots / group, Li = s->Li, Lj = s->Lj, hp = HP, RP = s->RP, off = s->q + 1;
+  int64_t ppl = (int64_t)group * s->tilesB * s->tileY * HP;
+  float* rpad = ratio ? s->rpad.as<float>() : nullptr;
+  void* args[] = {&part, &nparts, &Li, &Lj, &hp, &ppl, &lfsub, &hx_out, &rpad, &RP, &off};
+  MLF_CUDA(launch_pdl((const void*)k_reduce_ratio, ceil_div(LL, 32), 32 * kReduceGroups, args, 0, st));
   return MLF_OK;
 }
 

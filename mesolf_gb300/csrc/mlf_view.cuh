@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   float* dtab = taps + 4 * TTW;                                // [maxc][maxc]
   float* rowp = dtab + A.maxc * A.maxc;                        // [T][maxc]
 
-  // ---- zero the forward-input planes (halos must be zero), stage R
+  // ---- zero the forward-input planes (halos must be zero)
   {
     if (XIN) {
       const int n4 = A.XProws * A.XP / 4, total = A.slots * n4;
@@ -256,12 +256,6 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
         const int sl = i / n4;
         reinterpret_cast<float4*>(slot_base + sl * A.slot_floats)[i - sl * n4] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
-    }
-    if (BWD) {
-      const int nr = A.RProws * A.RP;
-      const float4* src = reinterpret_cast<const float4*>(A.rpad);
-      float4* dst = reinterpret_cast<float4*>(rs);
-      for (int i = tid; i < nr / 4; i += blockDim.x) dst[i] = src[i];
     }
   }
 
@@ -289,6 +283,17 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
       if (XIN) taps[TTW + j] = __ldg(A.wf + first * TT + i);
     }
     if (DT) view_d_rows<T>(A, first, lt, rowp);
+  }
+  // Everything above depends on the PSF alone and overlaps the end of the kernel before (the
+  // reduction that forms this view's ratio image); the rest reads what that kernel wrote.  The
+  // kernel after may be launched now: it waits here in turn.
+  pdl_launch_dependents();
+  pdl_wait();
+  if (BWD) {
+    const int nr = A.RProws * A.RP;
+    const float4* src = reinterpret_cast<const float4*>(A.rpad);
+    float4* dst = reinterpret_cast<float4*>(rs);
+    for (int i = tid; i < nr / 4; i += blockDim.x) dst[i] = src[i];
   }
   __syncthreads();
   if (s_stop) return;
@@ -509,7 +514,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
                                         : MLF_VIEW_TILE(T, MODE_BWDC, a.small);                 \
     ViewArgs v = a;                                                                             \
     void* args[] = {&v};                                                                        \
-    cudaError_t e = cudaLaunchKernel(f, dim3(grid), dim3(threads), args, smem, st);             \
+    cudaError_t e = launch_pdl(f, grid, threads, args, smem, st);                               \
     if (e != cudaSuccess)                                                                       \
       return fail(MLF_ERR_CUDA, std::string("view kernel launch: ") + cudaGetErrorString(e));   \
     return MLF_OK;                                                                              \
