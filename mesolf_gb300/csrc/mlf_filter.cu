@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "mlf_internal.h"
+#include "mlf_phase.cuh"
 
 namespace mlf {
 
@@ -26,53 +27,35 @@ constexpr int kPad = 33;        // shared-memory row stride (bank-conflict free)
 constexpr int kChunk = 8;       // consecutive outputs per thread
 constexpr int kFiltThreads = 512;
 constexpr int kLoadUnroll = 8;   // loads in flight per thread while staging lines
-constexpr int kRephaseLines = 4; // lines per block of k_rephase
 
+// The filter's scratch V: MATLAB layout with lines Vp = N*Pa floats apart (a multiple of 4, and the
+// volume's own size in all), so that eight outputs of a line are two 16-byte stores.
 struct FGeo {
-  int64_t Xr, Xc;
+  int64_t Xr, Xc, Vp;
   int Z;
 };
 
-// Offset in the phase-major volume X of the source of line (c, z) of the MATLAB layout
-// (length Xr = N*Li), element i enumerated as i = alpha*Li + a: that element is
-// line[N*a + alpha] = X[ch(alpha, beta, z)][b][a], beta = c mod N, b = c / N, so that
-// consecutive i read consecutive floats of one channel row.
-__device__ __forceinline__ int64_t line_src(const PatchGeo& g, int c, int z, int i) {
-  const int alpha = i / g.Li, a = i - alpha * g.Li;
-  return geo_channel(g, alpha, c % g.N, z) * g.plane + (int64_t)(c / g.N) * g.Pa + a;
-}
-
 // MATLAB layout -> phase-major for the filtered planes, scaling each plane by scale[z]: one
-// block per kRephaseLines lines (c, zlist[blockIdx.y]); the lines are staged in shared
-// memory so that both the read of V and the write of X's channel rows are coalesced.
-__global__ void k_rephase(const float* __restrict__ V, const double* __restrict__ scale,
+// block per kPhaseLines lines (c, zlist[blockIdx.y]), staged in shared memory (mlf_phase.cuh).
+__global__ void k_rephase(const float* __restrict__ V, FGeo f, const double* __restrict__ scale,
                           const int* __restrict__ zlist, PatchGeo g, float* __restrict__ X) {
-  extern __shared__ float lines[];  // [kRephaseLines][Xr]
-  const int c0 = blockIdx.x * kRephaseLines, z = zlist[blockIdx.y];
+  extern __shared__ __align__(16) float tab[];
+  float* const lines = tab + phase_tab_floats(g.N);  // [kPhaseLines][Xr]
+  const int c0 = blockIdx.x * kPhaseLines, z = zlist[blockIdx.y];
   const int Xr = (int)g.Xr;
-  const int nl = (int)(g.Xc - c0 < kRephaseLines ? g.Xc - c0 : kRephaseLines);
-  const int total = nl * Xr;
-  const float* src = V + ((int64_t)z * g.Xc + c0) * g.Xr;  // nl consecutive lines
-  for (int e0 = threadIdx.x; e0 < total; e0 += kLoadUnroll * blockDim.x) {
-    float v[kLoadUnroll];
+  const int nl = (int)(g.Xc - c0 < kPhaseLines ? g.Xc - c0 : kPhaseLines);
+  const float* src = V + ((int64_t)z * g.Xc + c0) * f.Vp;
+  for (int i = threadIdx.x; i < Xr; i += blockDim.x) {
+    float v[kPhaseLines];
 #pragma unroll
-    for (int u = 0; u < kLoadUnroll; ++u) {
-      const int e = e0 + u * blockDim.x;
-      v[u] = e < total ? src[e] : 0.f;
-    }
+    for (int l = 0; l < kPhaseLines; ++l) v[l] = l < nl ? src[l * f.Vp + i] : 0.f;
 #pragma unroll
-    for (int u = 0; u < kLoadUnroll; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e < total) lines[e] = v[u];
-    }
+    for (int l = 0; l < kPhaseLines; ++l) lines[l * Xr + i] = v[l];
   }
+  phase_table(g, c0, z, nl, 0, Xr, tab);
   __syncthreads();
   const double sc = scale[z];
-  for (int e = threadIdx.x; e < total; e += blockDim.x) {
-    const int l = e / Xr, i = e - l * Xr;
-    const int alpha = i / g.Li, a = i - alpha * g.Li;
-    X[line_src(g, c0 + l, z, i)] = (float)((double)lines[l * Xr + g.N * a + alpha] * sc);
-  }
+  phase_lines_out(X, g, nl, g.Li, tab, lines, [sc](float v) { return (float)((double)v * sc); });
 }
 
 // Circular 1-D filtering of kLines lines of length L held in shared memory as
@@ -83,7 +66,7 @@ __global__ void k_rephase(const float* __restrict__ V, const double* __restrict_
 // taps in groups of 8 over a 16-value register window, so one group costs 8 window loads
 // and 2 tap loads for 64 FMAs.  Every output adds its products in the order k = 0, 1, ...
 // (the zero taps add exactly nothing).
-// `emit(line, i, value)` stores an output; returns the thread's FP64 sum of outputs.
+// `emit(line, i0, values)` stores the outputs i0 .. i0 + 7 below L; returns the thread's FP64 sum of outputs.
 template <class Emit>
 __device__ double filter_lines(const float* __restrict__ buf, int L, const float* __restrict__ taps,
                                int ntp, int wlo, int nlines, Emit emit) {
@@ -126,14 +109,10 @@ __device__ double filter_lines(const float* __restrict__ buf, int L, const float
       jb -= 8;
       while (jb < 0) jb += L;
     }
+    emit(lane, i0, acc);
 #pragma unroll
-    for (int t = 0; t < kChunk; ++t) {
-      const int i = i0 + t;
-      if (i < L) {
-        emit(lane, i, acc[t]);
-        s += (double)acc[t];
-      }
-    }
+    for (int t = 0; t < kChunk; ++t)
+      if (i0 + t < L) s += (double)acc[t];
   }
   return s;
 }
@@ -161,8 +140,8 @@ __device__ void block_reduce_store(double s, double* out) {
 }
 
 // Pass along r: grid (ceil(Xc / kLines), Zf).  Lines = columns c of plane z, gathered
-// straight from the phase-major volume X (line_src); the row-filtered lines are written to
-// V in MATLAB layout.  Also accumulates the plane's input sum (sum_before).
+// straight from the phase-major volume X (mlf_phase.cuh); the row-filtered lines are written to
+// V.  Also accumulates the plane's input sum (sum_before).
 __global__ void k_filter_r(const float* __restrict__ X, PatchGeo pg, float* __restrict__ V, FGeo g,
                            const int* __restrict__ zlist, const int* __restrict__ plane_entry,
                            const float* __restrict__ cx, const int* __restrict__ wlo_e,
@@ -172,38 +151,19 @@ __global__ void k_filter_r(const float* __restrict__ X, PatchGeo pg, float* __re
   const int e = plane_entry[z];
   const int c0 = blockIdx.x * kLines;
   const int nlines = (int)(g.Xc - c0 < kLines ? g.Xc - c0 : kLines);
-  float* plane = V + (int64_t)z * g.Xr * g.Xc;
+  float* plane = V + (int64_t)z * g.Vp * g.Xc;
   const int L = (int)g.Xr;
   float* tsm = buf + taps_offset(L);
   const int ntp = stage_taps(tsm, cx + (int64_t)e * tap_stride, nt_e[e]);
-  // element e = l * L + i of the block's lines; 8 loads in flight per thread
   double sin = 0.0;
-  const int total = nlines * L;
-  for (int e0 = threadIdx.x; e0 < total; e0 += kLoadUnroll * blockDim.x) {
-    float v[kLoadUnroll];
-#pragma unroll
-    for (int u = 0; u < kLoadUnroll; ++u) {
-      const int e = e0 + u * blockDim.x;
-      v[u] = 0.f;
-      if (e < total) {
-        const int l = e / L;
-        v[u] = X[line_src(pg, c0 + l, z, e - l * L)];
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kLoadUnroll; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e < total) {
-        const int l = e / L, i = e - l * L;
-        const int alpha = i / pg.Li, a = i - alpha * pg.Li;
-        buf[(pg.N * a + alpha) * kPad + l] = v[u];
-        sin += (double)v[u];
-      }
-    }
-  }
+  phase_gather(X, pg, c0, z, nlines, 0, pg.Li, buf, kPad, 1, [&](float v) { sin += (double)v; });
   __syncthreads();
-  double sout = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines,
-                             [&](int l, int i, float y) { plane[(int64_t)(c0 + l) * g.Xr + i] = y; });
+  double sout = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
+    // the pitch holds whole groups of four; its floats past the line are never read
+    float* d = plane + (int64_t)(c0 + l) * g.Vp + i0;
+    *reinterpret_cast<float4*>(d) = make_float4(y[0], y[1], y[2], y[3]);
+    if (i0 + 4 < g.Vp) *reinterpret_cast<float4*>(d + 4) = make_float4(y[4], y[5], y[6], y[7]);
+  });
   (void)sout;
   block_reduce_store(sin, sums_in + (int64_t)blockIdx.y * gridDim.x + blockIdx.x);
 }
@@ -221,7 +181,7 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
   float* tsm = buf + taps_offset((int)g.Xc);
   const int ntp = stage_taps(tsm, cy + (int64_t)e * tap_stride, nt_e[e]);
   const int nlines = (int)(g.Xr - r0 < kLines ? g.Xr - r0 : kLines);
-  float* plane = V + (int64_t)z * g.Xr * g.Xc;
+  float* plane = V + (int64_t)z * g.Vp * g.Xc;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   // 8 column loads in flight per thread
   for (int c0 = warp; c0 < (int)g.Xc; c0 += kLoadUnroll * nwarps) {
@@ -229,7 +189,7 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
 #pragma unroll
     for (int u = 0; u < kLoadUnroll; ++u) {
       const int c = c0 + u * nwarps;
-      v[u] = (c < g.Xc && lane < nlines) ? plane[(int64_t)c * g.Xr + r0 + lane] : 0.f;
+      v[u] = (c < g.Xc && lane < nlines) ? plane[(int64_t)c * g.Vp + r0 + lane] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < kLoadUnroll; ++u) {
@@ -239,8 +199,11 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
   }
   __syncthreads();
   const int L = (int)g.Xc;
-  double s = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines,
-                          [&](int l, int i, float y) { plane[(int64_t)i * g.Xr + r0 + l] = y; });
+  double s = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
+#pragma unroll
+    for (int t = 0; t < kChunk; ++t)
+      if (i0 + t < L) plane[(int64_t)(i0 + t) * g.Vp + r0 + l] = y[t];
+  });
   block_reduce_store(s, sums_out + (int64_t)blockIdx.y * gridDim.x + blockIdx.x);
 }
 
@@ -431,7 +394,7 @@ int filter_run_geo(Solver* s, const PatchGeo& g, float* X, cudaStream_t st) {
   const int* nt_x = wlo_x + ne;
   const int* wlo_y = nt_x + ne;
   const int* nt_y = wlo_y + ne;
-  const FGeo fg{s->Xr, s->Xc, Z};
+  const FGeo fg{s->Xr, s->Xc, (int64_t)s->N * s->Pa, Z};
   float* V = s->Xtmp.as<float>();
   const int gr = (int)((s->Xc + kLines - 1) / kLines), gc = (int)((s->Xr + kLines - 1) / kLines);
   double* sin = f.sums.as<double>();
@@ -443,8 +406,9 @@ int filter_run_geo(Solver* s, const PatchGeo& g, float* X, cudaStream_t st) {
   k_filter_c<<<dim3(gc, nzf), kFiltThreads, sizeof(float) * ((size_t)taps_offset(Lc) + ((Lc + 7) & ~7)), st>>>(
       V, fg, zl, pe, f.cy.as<float>(), wlo_y, nt_y, Lc, sout);
   k_filter_scale<<<(Z + 255) / 256, 256, 0, st>>>(sin, gr, sout, gc, zl, nzf, Z, scale);
-  k_rephase<<<dim3((Lc + kRephaseLines - 1) / kRephaseLines, nzf), 256, sizeof(float) * kRephaseLines * Lr, st>>>(
-      V, scale, zl, g, X);
+  k_rephase<<<dim3((Lc + kPhaseLines - 1) / kPhaseLines, nzf), 256,
+              sizeof(float) * (phase_tab_floats(g.N) + kPhaseLines * Lr), st>>>(
+      V, fg, scale, zl, g, X);
   MLF_LAUNCHED();
   return MLF_OK;
 }
