@@ -28,8 +28,8 @@ constexpr int kChunk = 8;       // consecutive outputs per thread
 constexpr int kFiltThreads = 512;
 constexpr int kLoadUnroll = 8;   // loads in flight per thread while staging lines
 
-// The filter's scratch V: MATLAB layout with lines Vp = N*Pa floats apart (a multiple of 4, and the
-// volume's own size in all), so that eight outputs of a line are two 16-byte stores.
+// The filter's scratch V: MATLAB layout with lines Vp = filter_pitch(Xr) floats apart, a multiple of 4,
+// so that eight outputs of a line are two 16-byte stores.
 struct FGeo {
   int64_t Xr, Xc, Vp;
   int Z;
@@ -394,7 +394,7 @@ int filter_run_geo(Solver* s, const PatchGeo& g, float* X, cudaStream_t st) {
   const int* nt_x = wlo_x + ne;
   const int* wlo_y = nt_x + ne;
   const int* nt_y = wlo_y + ne;
-  const FGeo fg{s->Xr, s->Xc, (int64_t)s->N * s->Pa, Z};
+  const FGeo fg{s->Xr, s->Xc, filter_pitch(s->Xr), Z};
   float* V = s->Xtmp.as<float>();
   const int gr = (int)((s->Xc + kLines - 1) / kLines), gc = (int)((s->Xr + kLines - 1) / kLines);
   double* sin = f.sums.as<double>();

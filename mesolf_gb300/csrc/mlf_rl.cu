@@ -766,7 +766,7 @@ int solver_init(Solver* s) {
 
 int lite_prepare(Solver* s) {
   if (!s->lite || s->lite_ready) return MLF_OK;
-  MLF_TRY(s->Xtmp.alloc((size_t)s->N * s->Pa * s->Xc * s->Z * sizeof(float), "filter scratch"));
+  MLF_TRY(s->Xtmp.alloc((size_t)filter_pitch(s->Xr) * s->Xc * s->Z * sizeof(float), "filter scratch"));
   MLF_TRY(s->red.alloc(4096 * sizeof(double), "reduction scratch"));
   MLF_TRY(filter_init(s));
   s->lite_ready = true;
