@@ -174,6 +174,8 @@ struct Solver {
   int64_t nch = 0;
   // view-kernel geometry (tileY x tileX: the kernel's tile)
   bool small = false;  // the view kernel's small tile
+  bool fwd_xtwo = false;  // the forward kernel stages two X planes per slot
+  size_t fwd_smem = 0;    // ... its dynamic shared memory
   int tileY = 0, tileX = 0;
   int tilesA = 0, tilesB = 0, tps = 0, slots = 0, tstride = 0, threads = 0, grid = 0;
   int RP = 0, RProws = 0, XP = 0, XProws = 0, maxc = 0;
@@ -336,6 +338,7 @@ struct ViewArgs {
   int tilesA, tilesB, tps, slots, tstride;  // tstride: threads per slot (>= tps)
   int RP, RProws, XP, XProws, maxc, slot_floats;
   int small;           // the small tile
+  int xtwo;            // MODE_FWD: two X planes per slot (slot_floats holds both)
   CancelRef cancel;    // all null: not cancellable
 };
 enum ViewMode { MODE_FWD = 0, MODE_STEP = 1, MODE_BWDC = 2 };

@@ -338,6 +338,15 @@ ViewArgs view_args(Solver* s) {
   return a;
 }
 
+// One view kernel launch; the forward kernel has its own shared memory.
+int launch_view(Solver* s, int mode, ViewArgs a, cudaStream_t st) {
+  if (mode == MODE_FWD && s->fwd_xtwo) {
+    a.xtwo = 1;
+    a.slot_floats += s->XProws * s->XP;
+  }
+  return launch_view_kernel(s->T, mode, a, s->grid, s->threads, mode == MODE_FWD ? s->fwd_smem : s->smem, st);
+}
+
 const float* wf_of(const Solver* s, int view) {
   return s->psf->wf.as<float>() + (int64_t)view * s->psf->taps_per_view;
 }
@@ -423,7 +432,7 @@ int run_view(Solver* s, int mode, int view_cur, int view_next, float w, bool do_
   a.do_fwd = do_fwd ? 1 : 0;
   a.wb = wb_of(s, view_cur);
   a.wf = wf_of(s, view_next >= 0 ? view_next : view_cur);
-  MLF_TRY(launch_view_kernel(s->T, mode, a, s->grid, s->threads, s->smem, st));
+  MLF_TRY(launch_view(s, mode, a, st));
   return timing_mark(s, st);
 }
 
@@ -744,6 +753,12 @@ int solver_init(Solver* s) {
   int per_sm = 1;
   MLF_TRY(occupancy_view_kernel(s->T, s->small, s->threads, s->smem, &per_sm));
   per_sm = std::max(1, per_sm);
+  // the forward kernel stages no ratio image: a second X plane per slot where as many CTAs still fit
+  // (not with the small tile, whose launches are short: zeroing the plane costs what it hides)
+  const int xplane = s->XProws * s->XP;
+  const size_t two = sizeof(float) * (size_t)s->slots * (slot_floats + xplane);
+  s->fwd_xtwo = !s->small && two <= (size_t)dev_smem && (int64_t)per_sm * (int64_t)(two + 1024) <= sm_per_sm;
+  s->fwd_smem = s->fwd_xtwo ? two : sizeof(float) * (size_t)s->slots * slot_floats;
   const int64_t max_blocks = (s->nch + s->slots - 1) / s->slots;
   s->grid = (int)std::min<int64_t>(max_blocks, (int64_t)nsm * per_sm);
 
@@ -863,7 +878,7 @@ int forward_view(Solver* s, const float* d_vol, int u, int v, float* d_hx, cudaS
   a.u = u; a.v = v; a.w = 0.f; a.do_fwd = 1;
   a.wb = wb_of(s, u + s->N * v);
   a.wf = wf_of(s, u + s->N * v);
-  MLF_TRY(launch_view_kernel(s->T, MODE_FWD, a, s->grid, s->threads, s->smem, st));
+  MLF_TRY(launch_view(s, MODE_FWD, a, st));
   return run_reduce(s, u + s->N * v, d_hx, false, st);
 }
 
@@ -890,7 +905,7 @@ int forward_project(Solver* s, const float* d_vol, float* d_lf, const float* d_z
     a.u = view % N; a.v = view / N; a.w = 0.f; a.do_fwd = 1;
     a.wb = wb_of(s, view);
     a.wf = wf_of(s, view);
-    MLF_TRY(launch_view_kernel(s->T, MODE_FWD, a, s->grid, s->threads, s->smem, st));
+    MLF_TRY(launch_view(s, MODE_FWD, a, st));
     MLF_TRY(run_reduce(s, view, s->lfs.as<float>() + view * LL, false, st));
   }
   return launch_scatter_views(s->lfs.as<float>(), g, d_lf, LL, 0, st);
@@ -961,7 +976,7 @@ int backward_view(Solver* s, const float* d_proj, int u, int v, float* d_out, cu
   a.u = u; a.v = v; a.w = 0.f; a.do_fwd = 0;
   a.wb = wb_of(s, u + s->N * v);
   a.wf = wf_of(s, u + s->N * v);
-  MLF_TRY(launch_view_kernel(s->T, MODE_BWDC, a, s->grid, s->threads, s->smem, st));
+  MLF_TRY(launch_view(s, MODE_BWDC, a, st));
   return launch_from_phase(s->Xtmp.as<float>(), solver_geo(s), d_out, st);
 }
 

@@ -147,6 +147,10 @@ __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
   const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
@@ -211,6 +215,11 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   constexpr int QP = view_qpad(Q);      // column of the forward-input interior
   constexpr bool BWD = (MODE != MODE_FWD);
   constexpr bool XIN = (MODE != MODE_BWDC);
+  // The next channel's taps are requested at the start of a channel: 31 x 40 x 26 lenslets, T 9, forward
+  // 46.7 -> 43.4 us per view with the second X plane, 28 x 21 x 25, T 11 solve 20.0 -> 19.4 ms.  The
+  // small tile's few channels per slot gain nothing (11 x 11 x 21: 10.98 ms -> 11.05) and load them at
+  // the end.
+  constexpr bool AHEAD = TX == VW_TX;
   const int tid = threadIdx.x;
   const int slot = tid / A.tstride;          // slots start at multiples of tstride >= tps
   const int lt = tid - slot * A.tstride;     // thread index within slot
@@ -243,15 +252,19 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   // ---- shared memory carve-up
   float* rs = sm;                                              // [RProws][RP] (BWD only)
   float* slot_base = rs + (BWD ? A.RProws * A.RP : 0);
-  float* xin = slot_base + (slot_ok ? slot : 0) * A.slot_floats;  // [XProws][XP]
-  float* taps = xin + A.XProws * A.XP;                         // [2 buffers][wb | wf]
+  // forward only: two X planes where they fit, so that the next channel's loads overlap this one's
+  // projection (elsewhere they overlap the back projection)
+  const bool xtwo = MODE == MODE_FWD && AHEAD && A.xtwo;
+  const int xplane = A.XProws * A.XP;
+  float* xin = slot_base + (slot_ok ? slot : 0) * A.slot_floats;  // [1 or 2][XProws][XP]
+  float* taps = xin + (xtwo ? 2 : 1) * xplane;                 // [2 buffers][wb | wf]
   float* dtab = taps + 4 * TTW;                                // [maxc][maxc]
   float* rowp = dtab + A.maxc * A.maxc;                        // [T][maxc]
 
   // ---- zero the forward-input planes (halos must be zero)
   {
     if (XIN) {
-      const int n4 = A.XProws * A.XP / 4, total = A.slots * n4;
+      const int n4 = (xtwo ? 2 : 1) * xplane / 4, total = A.slots * n4;
       for (int i = tid; i < total; i += blockDim.x) {
         const int sl = i / n4;
         reinterpret_cast<float4*>(slot_base + sl * A.slot_floats)[i - sl * n4] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -273,15 +286,38 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
            (int64_t)b0 * HP + a0;
   };
   bool hx_written = false;
+  auto load_taps = [&](int ch, int b) {
+    float* dst = taps + b * 2 * TTW;
+    for (int i = lt; i < TT; i += A.tps) {
+      const int j = (i / T) * TW + i % T;
+      if (AHEAD) {
+        if (BWD) cp_async4(dst + j, A.wb + ch * TT + i);
+        if (XIN) cp_async4(dst + TTW + j, A.wf + ch * TT + i);
+      } else {
+        if (BWD) dst[j] = __ldg(A.wb + ch * TT + i);
+        if (XIN) dst[TTW + j] = __ldg(A.wf + ch * TT + i);
+      }
+    }
+  };
+  // X tile -> forward-input plane (interior at rows +Q, cols +QP).  A plane row has Pa (a multiple
+  // of 4) floats: a 16-byte chunk of the last tile may lie past it and is then not copied (its
+  // shared-memory cells stay zero).
+  auto load_x = [&](int ch, float* plane) {
+    const float* Xch = A.X + ch * A.plane;
+#pragma unroll
+    for (int y = 0; y < TY; ++y) {
+      const int b = b0 + y;
+      if (b >= A.Lj) continue;
+#pragma unroll
+      for (int k = 0; k < NC; ++k)
+        if (a0 + 4 * k < A.Pa) cp_async16(plane + (b + Q) * A.XP + xc[k], Xch + (int64_t)b * A.Pa + a0 + 4 * k);
+    }
+  };
 
   // taps of the first channel into buffer 0, its D row sums; the table after the barrier
   // (the row sums come from other threads)
   if (slot_ok && first < nch) {
-    for (int i = lt; i < TT; i += A.tps) {
-      const int j = (i / T) * TW + i % T;
-      if (BWD) taps[j] = __ldg(A.wb + first * TT + i);
-      if (XIN) taps[TTW + j] = __ldg(A.wf + first * TT + i);
-    }
+    load_taps(first, 0);
     if (DT) view_d_rows<T>(A, first, lt, rowp);
   }
   // Everything above depends on the PSF alone and overlaps the end of the kernel before (the
@@ -295,6 +331,11 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     float4* dst = reinterpret_cast<float4*>(rs);
     for (int i = tid; i < nr / 4; i += blockDim.x) dst[i] = src[i];
   }
+  if (xtwo) {
+    __syncthreads();  // the planes are zeroed
+    if (slot_ok && first < nch) load_x(first, xin);
+  }
+  if (AHEAD) cp_async_wait_all();
   __syncthreads();
   if (s_stop) return;
   if (DT && slot_ok && first < nch) view_d_table<T>(A, first, lt, rowp, dtab);
@@ -313,19 +354,13 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     const float* wbs = taps + buf * 2 * TTW;
     const float* wfs = wbs + TTW;
 
-    // ---- X tile -> forward-input plane (interior at rows +Q, cols +QP), asynchronously.
-    // A plane row has Pa (a multiple of 4) floats: a 16-byte chunk of the last tile may
-    // lie past it and is then not copied (its shared-memory cells stay zero).
-    if (XIN && active) {
-      const float* Xch = A.X + ch * A.plane;
-#pragma unroll
-      for (int y = 0; y < TY; ++y) {
-        const int b = b0 + y;
-        if (b >= A.Lj) continue;
-#pragma unroll
-        for (int k = 0; k < NC; ++k)
-          if (a0 + 4 * k < A.Pa) cp_async16(xin + (b + Q) * A.XP + xc[k], Xch + (int64_t)b * A.Pa + a0 + 4 * k);
-      }
+    // this channel's X (or, with two planes, the next one's) and the next channel's taps,
+    // asynchronously: the buffers they go to were last read before the barrier at the loop's end
+    float* const xcur = xin + (xtwo ? buf * xplane : 0);
+    if (XIN && active && !xtwo) load_x(ch, xin);
+    if (more) {
+      if (AHEAD) load_taps(nxt, buf ^ 1);
+      if (xtwo) load_x(nxt, xin + (buf ^ 1) * xplane);
     }
 
     // One correlation call site for both phases (back projection of view k, forward
@@ -334,7 +369,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
     for (int ph = 0; ph < 2; ++ph) {
       if (ph == 1 && !(XIN && (MODE == MODE_FWD || A.do_fwd))) break;
       if (active && ph == 0 && !BWD) {
-        cp_async_wait_all();  // forward only: this thread's X tile has landed in xin
+        if (!xtwo) cp_async_wait_all();  // forward only: this thread's X tile has landed in xin
       } else if (active) {
         float acc[TY][TX];
 #pragma unroll
@@ -347,7 +382,7 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
           for (int y = 0; y < TY; ++y)
             asm volatile("prefetch.global.L1 [%0];" ::"l"(hxp + y * A.tilesA * TX));
         }
-        const float* in = ph == 0 ? rs + (b0 + sb + 1) * A.RP : xin + b0 * A.XP;
+        const float* in = ph == 0 ? rs + (b0 + sb + 1) * A.RP : xcur + b0 * A.XP;
         const int pitch = ph == 0 ? A.RP : A.XP;
         const float* wsel = ph == 0 ? wbs : wfs;
         switch (ph == 0 ? sa + 1 : QP - Q) {
@@ -448,19 +483,12 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
         // the next channel's D row sums (global taps) while other warps still correlate;
         // the table below reads them after the barrier, once dtab has been read
         if (DT && more) view_d_rows<T>(A, nxt, lt, rowp);
-        __syncthreads();
+        if (!xtwo) __syncthreads();
       }
     }
-    // the next channel: its D table and its taps (into the other buffer)
-    if (more) {
-      if (DT) view_d_table<T>(A, nxt, lt, rowp, dtab);
-      float* nb = taps + (buf ^ 1) * 2 * TTW;
-      for (int i = lt; i < TT; i += A.tps) {
-        const int j = (i / T) * TW + i % T;
-        if (BWD) nb[j] = __ldg(A.wb + nxt * TT + i);
-        if (XIN) nb[TTW + j] = __ldg(A.wf + nxt * TT + i);
-      }
-    }
+    if (DT && more) view_d_table<T>(A, nxt, lt, rowp, dtab);  // the next channel's D table
+    if (!AHEAD && more) load_taps(nxt, buf ^ 1);
+    if (AHEAD) cp_async_wait_all();
     __syncthreads();
   }
 
