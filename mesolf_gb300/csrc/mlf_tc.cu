@@ -578,7 +578,9 @@ struct TcFwdArgs {
   float* ypart;  // [split][NB][MP] (tap-major: col2im reads it coalesced)
   int* err;
   int stages;    // shared-memory ring depth (2..FWD_MAX_STAGES)
-  int MP, NB, NH, nparts, splits, KS, frow0;  // frow0 = view * NB
+  int MP, NB, NH, nparts, splits, KS, frow0;  // MP: positions of ypart; frow0 = view * NB
+  int tile0;               // position tile of blockIdx.x = 0 (the first position of ypart)
+  int64_t vstride;         // blockIdx.z: views from the launch's first on, ypart vstride floats apart
   int use_alo, use_blo;                             // activation / tap hi+lo splits
   const float* wview;      // per patch weight of the projected view (nullable: project all)
   const int* tile_patch;   // patch of each position tile
@@ -606,7 +608,8 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
          const __grid_constant__ CUtensorMap mBl, TcFwdArgs a) {
   // a patch that does not use this view needs no projection for it (whole CTA, before any
   // barrier or TMEM allocation)
-  if (a.wview && __ldg(a.wview + __ldg(a.tile_patch + blockIdx.x)) == 0.f) return;
+  const int tile = a.tile0 + blockIdx.x, view = blockIdx.z;
+  if (a.wview && __ldg(a.wview + __ldg(a.tile_patch + tile)) == 0.f) return;
   {  // a cancelled solve: the rest of its view steps return at once (CTA-uniform, before TMEM)
     __shared__ int s_stop;
     if (threadIdx.x == 0) s_stop = cancel_entry(a.cancel);
@@ -620,10 +623,10 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
   __shared__ uint32_t tmem_base;
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.x * BM;
+  const int m0 = tile * BM, frow0 = a.frow0 + view * a.NB;
   const int split = blockIdx.y;
   // this split's channel blocks, clipped to the patch's planes (an empty range writes zeros)
-  const int* pq = a.pinfo + 8 * __ldg(a.tile_patch + blockIdx.x);
+  const int* pq = a.pinfo + 8 * __ldg(a.tile_patch + tile);
   const SplitRange sr = split_range(__ldg(pq + 4), __ldg(pq + 5), a.NN, a.splits, split, a.KS);
   const int ks0 = sr.ks0, ks1 = sr.ks1;
   const int tileB = a.NB * 128;  // NB rows x 128 bytes
@@ -665,9 +668,9 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
       tc::mbar_arrive_expect_tx(&full[s], bytes);
       tc::tma_load_2d(st, &mX, &full[s], m0, ks * BK);
       for (int p = 0; p < a.nparts; ++p) {
-        tc::tma_load_2d(st + offBh + p * a.NH * 128, &mBh, &full[s], ks * BK, a.frow0 + p * a.NH);
+        tc::tma_load_2d(st + offBh + p * a.NH * 128, &mBh, &full[s], ks * BK, frow0 + p * a.NH);
         if (a.use_blo)
-          tc::tma_load_2d(st + offBl + p * a.NH * 128, &mBl, &full[s], ks * BK, a.frow0 + p * a.NH);
+          tc::tma_load_2d(st + offBl + p * a.NH * 128, &mBl, &full[s], ks * BK, frow0 + p * a.NH);
       }
       ++issued;
     }
@@ -756,7 +759,7 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    float* out = a.ypart + (int64_t)split * a.NB * a.MP + m0 + row;  // + t * MP
+    float* out = a.ypart + view * a.vstride + (int64_t)split * a.NB * a.MP + blockIdx.x * BM + row;  // + t * MP
     const bool empty_split = ks1 <= ks0;
     // FP16: remove the volume's and the tap column's scales (powers of two: exact)
     const float xinv = F16 ? 1.f / f16_scale(*a.xmax) : 1.f;
@@ -767,7 +770,7 @@ k_tc_fwd(const __grid_constant__ CUtensorMap mX, const __grid_constant__ CUtenso
         if (aborted(&abort_flag)) continue;
         if (F16) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] *= xinv * __ldg(a.fsinv + c * 16 + j);
+          for (int j = 0; j < 16; ++j) v[j] *= xinv * __ldg(a.fsinv + view * a.NB + c * 16 + j);
         }
 #pragma unroll
         for (int j = 0; j < 16; ++j) out[(int64_t)(c * 16 + j) * a.MP] = empty_split ? 0.f : v[j];
@@ -1504,16 +1507,23 @@ k_tc_im2col(const float* __restrict__ R, const int* __restrict__ tile_patch, con
 // with eight and 17 with sixteen for 59136 positions with one split, 18.7 -> 7.9 for 3200 with six.  Sums in a fixed order
 // (deterministic).  rmax (nullable, FP16 modes) receives max |R|.
 constexpr int COL2IM_WARPS = 16;
+// The positions from pos0 on that ypart holds (MP of them), of the views blockIdx.y: their partials
+// vstride and their outputs hx_stride floats apart.
+struct PartRange {
+  int pos0;
+  int64_t vstride, hx_stride;
+};
 __global__ void __launch_bounds__(32 * COL2IM_WARPS)
 k_tc_col2im_ratio(const float* __restrict__ ypart, int splits, int MP, int NB, int T,
                   const int* __restrict__ tile_patch, const int* __restrict__ pinfo,
                   const float* __restrict__ lfsub, float* __restrict__ hx_out, float* __restrict__ rimg,
-                  float* __restrict__ rmax) {
+                  float* __restrict__ rmax, PartRange pr) {
   __shared__ float part[COL2IM_WARPS][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pos = blockIdx.x * 32 + lane;
+  const int pos = pr.pos0 + blockIdx.x * 32 + lane;
+  ypart += blockIdx.y * pr.vstride;
   float s = 0.f;
-  bool valid = pos < MP;
+  bool valid = pos - pr.pos0 < MP;
   int pos0 = 0, Li = 1, Lj = 0, j = 0, i = 0;
   if (valid) {
     const int* pi = pinfo + 8 * tile_patch[pos / BM];
@@ -1533,7 +1543,7 @@ k_tc_col2im_ratio(const float* __restrict__ ypart, int splits, int MP, int NB, i
       const int b = j + db - q;
       if (b < 0 || b >= Lj) continue;
       // element (db, da): (db*T + da)*MP + pos0 + b*Li + i + da - q
-      const float* yrow = ypart + (int64_t)(db * T) * MP + pos0 + (int64_t)b * Li + (i - q);
+      const float* yrow = ypart + (int64_t)(db * T) * MP + (pos0 - pr.pos0) + (int64_t)b * Li + (i - q);
       for (int sp = 0; sp < splits; ++sp, yrow += sstride) {
         for (int d0 = 0; d0 < T; d0 += 16) {
           float v[16];
@@ -1554,7 +1564,7 @@ k_tc_col2im_ratio(const float* __restrict__ ypart, int splits, int MP, int NB, i
     float h = 0.f;
 #pragma unroll
     for (int k = 0; k < COL2IM_WARPS; ++k) h += part[k][lane];
-    if (hx_out) hx_out[pos] = h;
+    if (hx_out) hx_out[blockIdx.y * pr.hx_stride + pos] = h;
     if (rimg) {
       float r = lfsub[pos] / h;
       if (!isfinite(r)) r = 0.f;
@@ -2012,15 +2022,22 @@ PatchGeo work_geo(const TcSolverState* t, const Solver* m, int p) {
 }
 
 // wview (nullable): per-patch weights of `view`; patches with weight 0 are not projected.
+// A forward GEMM and its col2im: position tiles [tile0, tile0 + ntiles) (whole patches) of nviews views.
+struct TcPart {
+  int tile0 = 0, ntiles = 0, nviews = 1;  // ntiles 0: all
+};
 int tc_fwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, cudaStream_t st,
-                  const float* wview = nullptr, bool cancellable = false) {
+                  const float* wview = nullptr, bool cancellable = false, TcPart part = TcPart()) {
   const TcPsfState* tp = psf->tc;
   int alo, blo;
   splits_of(precision, &alo, &blo);
   TcFwdArgs a{};
   a.ypart = t->ypart.as<float>();
   a.err = t->err.as<int>();
-  a.MP = t->MP;
+  const int ntiles = part.ntiles ? part.ntiles : t->MP / BM;
+  a.MP = ntiles * BM;
+  a.tile0 = part.tile0;
+  a.vstride = (int64_t)t->splits * tp->NB * a.MP;
   a.NB = tp->NB;
   a.NH = tp->NH;
   a.nparts = tp->nparts;
@@ -2046,20 +2063,22 @@ int tc_fwd_launch(const Psf* psf, TcSolverState* t, int precision, int view, cud
   if (fsmem > (size_t)tp->fwd_dyn_max)
     return fail(MLF_ERR_UNSUPPORTED, "tensor-core forward projection: taps tile exceeds shared memory");
   if (use16)
-    k_tc_fwd<true><<<dim3(t->MP / BM, t->splits), FWD_THREADS, fsmem, st>>>(t->mXv, tp->mFh16, tp->mFl16, a);
+    k_tc_fwd<true><<<dim3(ntiles, t->splits, part.nviews), FWD_THREADS, fsmem, st>>>(t->mXv, tp->mFh16, tp->mFl16, a);
   else
-    k_tc_fwd<false><<<dim3(t->MP / BM, t->splits), FWD_THREADS, fsmem, st>>>(t->mXv, tp->mFh, tp->mFl, a);
+    k_tc_fwd<false><<<dim3(ntiles, t->splits, part.nviews), FWD_THREADS, fsmem, st>>>(t->mXv, tp->mFh, tp->mFl, a);
   MLF_LAUNCHED();
   return MLF_OK;
 }
 
 // slot (FP16 modes): the max |R| slot of this view step (its parity within the iteration)
 int tc_col2im(const Psf* psf, TcSolverState* t, int view, bool ratio, float* hx_out, cudaStream_t st,
-              int precision = MLF_PREC_BF16X2, int slot = 0) {
+              int precision = MLF_PREC_BF16X2, int slot = 0, TcPart part = TcPart()) {
+  const int MP = (part.ntiles ? part.ntiles : t->MP / BM) * BM;
+  const PartRange pr{part.tile0 * BM, (int64_t)t->splits * psf->tc->NB * MP, t->MP};
   float* rmax = (ratio && prec_f16(precision)) ? t->f16s.as<float>() + 1 + slot : nullptr;
-  k_tc_col2im_ratio<<<(t->MP + 31) / 32, 32 * COL2IM_WARPS, 0, st>>>(
-      t->ypart.as<float>(), t->splits, t->MP, psf->tc->NB, psf->T, t->tile_patch.as<int>(), t->pinfo.as<int>(),
-      t->lfs.as<float>() + (int64_t)view * t->MP, hx_out, ratio ? t->rimg.as<float>() : nullptr, rmax);
+  k_tc_col2im_ratio<<<dim3((MP + 31) / 32, part.nviews), 32 * COL2IM_WARPS, 0, st>>>(
+      t->ypart.as<float>(), t->splits, MP, psf->tc->NB, psf->T, t->tile_patch.as<int>(), t->pinfo.as<int>(),
+      t->lfs.as<float>() + (int64_t)view * t->MP, hx_out, ratio ? t->rimg.as<float>() : nullptr, rmax, pr);
   MLF_LAUNCHED();
   return MLF_OK;
 }
@@ -2595,10 +2614,30 @@ int tc_forward_project(TcSolverState* t, const std::vector<Solver*>& members, co
     MLF_TRY(launch_to_phase(vols[p], work_geo(t, members[p], p), t->X.as<float>() + t->pos0[p], st,
                             zscale ? zscale + t->z0[p] : nullptr));
   MLF_TRY(tc_f16_begin(t, precision, st));
-  for (int view = 0; view < N * N; ++view) {
-    MLF_TRY(tc_fwd_launch(psf, t, precision, view, st));
-    MLF_TRY(tc_col2im(psf, t, view, false, t->lfs.as<float>() + (int64_t)view * t->MP, st));
+  // The GEMM runs one CTA per SM, a view's tiles in waves.  A last wave that fills less than half the
+  // SMs is left out of the views: its patches follow for as many views in one launch as fill whole
+  // waves, in the same partials buffer.  376 x 376 x 77 slices, kw 241: 462 tiles on 152 SMs, the last 6
+  // alone took a quarter of the GEMM's time: 21.1 -> 18.9 ms per call.
+  const int tiles = t->MP / BM, waves = tiles / t->nsm, rest = tiles % t->nsm;
+  TcPart main{0, tiles, 1}, tail{0, 0, 0};
+  if (t->splits == 1 && waves > 0 && rest > 0 && 2 * rest <= t->nsm) {
+    int cut = 0;  // the last patch boundary inside the full waves
+    for (int p = 0; p < t->P; ++p)
+      if (t->pos0[p] / BM <= tiles - rest) cut = (int)(t->pos0[p] / BM);
+    const int left = tiles - cut;
+    if (cut > 0 && 2 * left <= t->nsm) {
+      main.ntiles = cut;
+      tail = TcPart{cut, left, waves * t->nsm / left};
+    }
   }
+  auto project = [&](TcPart part, int view) -> int {
+    part.nviews = std::min(part.nviews, N * N - view);
+    MLF_TRY(tc_fwd_launch(psf, t, precision, view, st, nullptr, false, part));
+    return tc_col2im(psf, t, view, false, t->lfs.as<float>() + (int64_t)view * t->MP, st, MLF_PREC_BF16X2, 0, part);
+  };
+  for (int view = 0; view < N * N; ++view) MLF_TRY(project(main, view));
+  if (tail.nviews)
+    for (int view = 0; view < N * N; view += tail.nviews) MLF_TRY(project(tail, view));
   for (int p = 0; p < t->P; ++p)
     MLF_TRY(launch_scatter_views(t->lfs.as<float>(), work_geo(t, members[p], p), lf_out[p], t->MP, t->pos0[p], st));
   return MLF_OK;
