@@ -10,27 +10,28 @@
 // treated as zero here too.
 //
 // Direct kernel (k_conv_vec_lanes).  The outputs of one row phase b = y % 15 share one set of
-// 15 kernels (one per x phase).  A thread owns a segment of 15 consecutive outputs
-// x = 15 i + a, a = 0..14 -- one per x phase -- in RPT rows y = b + 15 j of one slice; the
-// (slice, row group, segment) triples of a phase are the lanes of its CTAs, so warps are full
-// whatever the sizes.  Per kernel row ky a CTA stages the input rows its lanes read and the 15
-// kernels' row ky ([kx][a], padded to 16) in shared memory with zero-filling cp.async, double
-// buffered so that row ky + 1 loads while row ky is computed.  Along kx the thread slides a window
-// of 15 inputs per row in registers (one new shared load per step and row) and reads the step's
-// 15 taps as broadcast 16-byte loads; kw is padded to a multiple of 15 with zero taps so that the
-// 15-step rotation of the window needs no tail.  Every output adds its products in the
+// 15 kernels (one per x phase).  A thread owns SEG consecutive outputs x = 15 i + a of a segment of
+// 15 -- all its x phases a, or one half of them (a = 0..7 or 8..14, a CTA's threads the same half) --
+// in RPT rows y = b + 15 j of one slice; the (slice, row group, segment) triples of a phase are the
+// lanes of its CTAs, so warps are full whatever the sizes.  Per kernel row ky a CTA stages the input
+// rows its lanes read and its kernels' row ky ([kx][a], padded to 16 or 8) in shared memory with
+// zero-filling cp.async, double buffered so that row ky + 1 loads while row ky is computed.  Along kx
+// the thread slides a window of inputs per row in registers (one new shared load per step and row)
+// and reads the step's taps as broadcast 16-byte loads.  Whole segments: kw is padded to a multiple
+// of 15 with zero taps so that the 15-step rotation of the window needs no tail.  Every output adds its products in the
 // reference's order -- kernel rows in order, each row left to right, one FP32 FMA chain
 // (mex_lfm_convolution_vec.cu:147-251) -- and the products it adds beyond the reference's
 // clipped window multiply zero-filled inputs, which adds exactly 0 for finite kernels; so
 // the output equals the reference kernel's bit for bit (tests/test_gpu_ref_mex.py).
 //
-// Bound: small calls have fewer warps than the chip has schedulers, so there one row per thread
-// spreads the work over the SMs; where the SMs are full, the shared-memory pipe, which returns a
-// step's taps to every warp (four 16-byte loads, 512 bytes each, for 15 FMAs per row): two rows
-// share them.  The columns that a row has off the image are zeroed once, so staging copies what
-// the image has and needs no test per element.  253 x 198 x 4, kw 136: 1.15 -> 0.60 ms (the
-// previous form launched 60 CTAs); 396 x 380 x 9, kw 151: 2.56 -> 2.07; 376 x 376 x 77, kw 241:
-// 45.2 -> 33.9 ms (37 TFLOP/s).
+// Bound: small calls have fewer warps than the chip has schedulers, and a lone warp spends 2.5 cycles
+// per instruction, so there one row and half a segment per thread give twice the warps for the same
+// instructions per FMA; where the SMs are full, the shared-memory pipe, which returns a step's taps to
+// every warp (two wavefronts per broadcast 16-byte load): two rows of a whole segment share four.
+// The columns that a row has off the image are zeroed once, so staging copies what the image has and
+// needs no test per element.  Half segments against one row of a whole segment: 253 x 198 x 4, kw 136
+// 571 -> 483 us, 33 x 200 x 1, kw 241 1486 -> 765, 40 x 35 x 2, kw 21 54 -> 38; two rows of a whole
+// segment: 396 x 380 x 9, kw 151 2.07 ms, 376 x 376 x 77, kw 241 33.9 ms (37 TFLOP/s).
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -42,6 +43,9 @@ namespace mlf {
 namespace {
 
 constexpr int CV_NN = 15;           // kernels per axis (the reference's num_kernels)
+constexpr int CV_HALF = 8;           // x phases of the first half of a segment (the second has 7)
+constexpr int CV_RING = 2 * CV_HALF; // half segments: inputs of a row held in registers
+constexpr int CV_TAHEAD = 2;         // ... kernel columns whose taps are
 constexpr int CV_MAX_THREADS = 384;  // 12 warps of up to 168 registers
 constexpr int CV_MAX_ROWS = 512;    // staged rows per CTA
 
@@ -57,7 +61,7 @@ struct ConvArgs {
   const float* K;    // kw x kw x 15 x 15 (kx fastest; kernel (a, b) at kw*kw*(a + 15 b))
   float* out;
   int W, H, kw, hk, Wv, Hv;  // Wv, Hv: columns / rows that can contribute (even kw: W-1, H-1)
-  int kwp;                   // kw rounded up to a multiple of 15 (the extra taps are zero)
+  int kwp;                   // kernel columns walked: kw, or with whole segments the next multiple of 15 (zero taps)
   int SX, tilesX;            // segments per group and groups along x
   int width, pitch, gstride; // staged row: width = 15 SX + kwp - 1 floats, pitch apart; a group's RPT rows gstride
   int max_groups;            // groups that a CTA's lanes can touch
@@ -65,13 +69,18 @@ struct ConvArgs {
 };
 
 // Lane l of phase b: group l / SX = (slice * nP + row group) * tilesX + x tile, segment l % SX.
-template <int RPT>
+// SEG 15: blockIdx.y is the phase; SEG CV_HALF: 2 * phase + half.
+template <int RPT, int SEG>
 __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
+  constexpr bool HALF = SEG != CV_NN;
+  constexpr int TP = HALF ? CV_HALF : 16;     // floats per kernel column of the staged taps
   extern __shared__ __align__(16) float sm[];
   __shared__ int row_y[CV_MAX_ROWS];          // staged row: image row at ky = 0 (INT_MIN / 2: none)
   __shared__ int64_t row_src[CV_MAX_ROWS];    // ... its offset, at the tile's first column
   __shared__ short2 row_col[CV_MAX_ROWS];     // ... staged columns [x, y) that the image has
-  const int b = blockIdx.y;                   // row phase
+  const int b = HALF ? blockIdx.y >> 1 : blockIdx.y;        // row phase
+  const int a0 = HALF ? (blockIdx.y & 1) * CV_HALF : 0;     // first x phase
+  const int na = HALF && a0 ? CV_NN - CV_HALF : SEG;        // x phases
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int nJ = b < A.H ? (A.H - b + CV_NN - 1) / CV_NN : 0;  // rows of this phase
   const int nP = (nJ + RPT - 1) / RPT;
@@ -93,7 +102,7 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
     const int j = jp * RPT + rr % RPT;
     const int y0 = b + CV_NN * j - A.hk;
     row_y[rr] = j < nJ ? y0 : INT_MIN / 2;
-    const int c0 = CV_NN * A.SX * xt - A.hk;
+    const int c0 = CV_NN * A.SX * xt + a0 - A.hk;
     const int ca = min(max(-c0, 0), A.width), cb = max(min(A.Wv - c0, A.width), ca);
     row_col[rr] = make_short2((short)ca, (short)cb);
     row_src[rr] = slice * (int64_t)A.W * A.H + (int64_t)y0 * A.W + c0;
@@ -105,9 +114,9 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
   const int il = active ? (int)(lane_id - g * A.SX) : 0;
   int jp, xt;
   const int64_t slice = group(g, jp, xt);
-  const int x_seg = CV_NN * (xt * A.SX + il);
+  const int x_seg = CV_NN * (xt * A.SX + il) + a0;
   const int rowbuf = A.max_groups * A.gstride;
-  float* const rows0 = sm + 32 * A.kwp;  // taps of buffer s at sm + 16 kwp s, rows at rows0 + rowbuf s
+  float* const rows0 = sm + 2 * TP * A.kwp;  // taps of buffer s at sm + TP kwp s, rows at rows0 + rowbuf s
   const int64_t kplane = (int64_t)A.kw * A.kw;
   const float* kb = A.K + kplane * CV_NN * b;  // kernels (a, b), a = 0..14
 
@@ -115,12 +124,12 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
   // off the image is zeroed where the buffer may hold another one.
   const int warp = tid >> 5, lane = tid & 31, nwarps = nthr >> 5;
   auto stage = [&](int ky, int s) {
-    float* tb = sm + s * 16 * A.kwp;
-    const int ta = tid & 15;
-    if (ta < CV_NN) {
-      const float* src = kb + kplane * ta + (int64_t)A.kw * ky;
+    float* tb = sm + s * TP * A.kwp;
+    const int ta = tid & (TP - 1);
+    if (ta < na) {
+      const float* src = kb + kplane * (a0 + ta) + (int64_t)A.kw * ky;
 #pragma unroll 4
-      for (int kx = tid >> 4; kx < A.kw; kx += nthr >> 4) cp_async4(tb + 16 * kx + ta, src + kx);
+      for (int kx = tid / TP; kx < A.kw; kx += nthr / TP) cp_async4(tb + TP * kx + ta, src + kx);
     }
     float* rb = rows0 + s * rowbuf;
     for (int rr = warp; rr < ng * RPT; rr += nwarps) {
@@ -138,18 +147,23 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
     cp_async_commit();
   };
   // the padding taps are zero in both buffers; nothing writes them again
-  for (int e = tid; e < 2 * 16 * (A.kwp - A.kw); e += nthr) {
-    const int s = e / (16 * (A.kwp - A.kw)), k = e - s * 16 * (A.kwp - A.kw);
-    sm[s * 16 * A.kwp + 16 * A.kw + k] = 0.f;
+  if (HALF) {  // the eighth phase of the second half
+    if (a0)
+      for (int e = tid; e < 2 * A.kwp; e += nthr) sm[TP * e + TP - 1] = 0.f;
+  } else {
+    for (int e = tid; e < 2 * TP * (A.kwp - A.kw); e += nthr) {
+      const int s = e / (TP * (A.kwp - A.kw)), k = e - s * TP * (A.kwp - A.kw);
+      sm[s * TP * A.kwp + TP * A.kw + k] = 0.f;
+    }
   }
   for (int e = tid; e < 2 * rowbuf; e += nthr) rows0[e] = 0.f;
   __syncthreads();  // the row table; the zeroed buffers
 
-  float acc[RPT][CV_NN];
+  float acc[RPT][SEG];
 #pragma unroll
   for (int r = 0; r < RPT; ++r)
 #pragma unroll
-    for (int a = 0; a < CV_NN; ++a) acc[r][a] = 0.f;
+    for (int a = 0; a < SEG; ++a) acc[r][a] = 0.f;
   stage(0, 0);
   cp_async_wait0();
   __syncthreads();
@@ -158,38 +172,77 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
     if (ky + 1 < A.kw) stage(ky + 1, sel ^ 1);
     if (active) {
       const float* rowp = rows0 + sel * rowbuf + (int)(g - g0) * A.gstride + CV_NN * il;
-      const float* tp = sm + sel * 16 * A.kwp;
-      float w[RPT][CV_NN];  // w[r][(m + a) % 15] holds row r at kx0 + m + a
-#pragma unroll
-      for (int r = 0; r < RPT; ++r)
-#pragma unroll
-        for (int a = 0; a < CV_NN - 1; ++a) w[r][a] = rowp[r * A.pitch + a];
+      const float* tp = sm + sel * TP * A.kwp;
       const float4* t4 = reinterpret_cast<const float4*>(tp);
-      float4 tc[4];  // taps of the step in work; the next step's load during it
+      if constexpr (HALF) {
+        // Rings of registers: slot k % 16 of the window holds the row's value at column k, slot
+        // k % CV_TAHEAD of the taps those of kernel column k.  A slot is loaded again as soon as it is
+        // used; the loads past the last column (other data of this CTA's shared memory) are not used.
+        float w[RPT][CV_RING];
+        float4 tq[CV_TAHEAD][2];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) tc[q] = t4[q];
+        for (int k = 0; k < CV_TAHEAD; ++k)
 #pragma unroll
-      for (int r = 0; r < RPT; ++r) w[r][CV_NN - 1] = rowp[r * A.pitch + CV_NN - 1];
+          for (int q = 0; q < 2; ++q) tq[k][q] = t4[2 * k + q];
+#pragma unroll
+        for (int k = 0; k < CV_RING; ++k)
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) w[r][k] = rowp[r * A.pitch + k];
+        auto column = [&](int kx0, int m) {
+          const float4 u = tq[m % CV_TAHEAD][0], v = tq[m % CV_TAHEAD][1];
+          const float t[CV_HALF] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int a = 0; a < SEG; ++a)
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) acc[r][a] = fmaf(w[r][(m + a) % CV_RING], t[a], acc[r][a]);
+#pragma unroll
+          for (int q = 0; q < 2; ++q) tq[m % CV_TAHEAD][q] = t4[2 * (kx0 + m + CV_TAHEAD) + q];
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) w[r][m] = rowp[r * A.pitch + kx0 + m + CV_RING];
+        };
+        int kx0 = 0;
 #pragma unroll 1
-      for (int kx0 = 0; kx0 < A.kwp; kx0 += CV_NN) {
+        for (; kx0 + CV_RING <= A.kwp; kx0 += CV_RING) {
 #pragma unroll
-        for (int m = 0; m < CV_NN; ++m) {
-          float4 tn[4];
+          for (int m = 0; m < CV_RING; ++m) column(kx0, m);
+        }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) tn[q] = t4[4 * (kx0 + m + 1) + q];  // past the last step: not used
-          float wn[RPT];
+        for (int m = 0; m < CV_RING - 1; ++m) {  // the remaining columns
+          if (kx0 + m >= A.kwp) break;
+          column(kx0, m);
+        }
+      } else {
+        float w[RPT][CV_NN];  // w[r][(m + a) % 15] holds row r at kx0 + m + a
 #pragma unroll
-          for (int r = 0; r < RPT; ++r) wn[r] = rowp[r * A.pitch + kx0 + m + CV_NN];
-          const float t[16] = {tc[0].x, tc[0].y, tc[0].z, tc[0].w, tc[1].x, tc[1].y, tc[1].z, tc[1].w,
-                               tc[2].x, tc[2].y, tc[2].z, tc[2].w, tc[3].x, tc[3].y, tc[3].z, tc[3].w};
+        for (int r = 0; r < RPT; ++r)
 #pragma unroll
-          for (int a = 0; a < CV_NN; ++a)
+          for (int a = 0; a < CV_NN - 1; ++a) w[r][a] = rowp[r * A.pitch + a];
+        float4 tc[4];  // taps of the step in work; the next step's load during it
 #pragma unroll
-            for (int r = 0; r < RPT; ++r) acc[r][a] = fmaf(w[r][(m + a) % CV_NN], t[a], acc[r][a]);
+        for (int q = 0; q < 4; ++q) tc[q] = t4[q];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) tc[q] = tn[q];
+        for (int r = 0; r < RPT; ++r) w[r][CV_NN - 1] = rowp[r * A.pitch + CV_NN - 1];
+#pragma unroll 1
+        for (int kx0 = 0; kx0 < A.kwp; kx0 += CV_NN) {
 #pragma unroll
-          for (int r = 0; r < RPT; ++r) w[r][m] = wn[r];
+          for (int m = 0; m < CV_NN; ++m) {
+            float4 tn[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tn[q] = t4[4 * (kx0 + m + 1) + q];  // past the last step: not used
+            float wn[RPT];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) wn[r] = rowp[r * A.pitch + kx0 + m + CV_NN];
+            const float t[16] = {tc[0].x, tc[0].y, tc[0].z, tc[0].w, tc[1].x, tc[1].y, tc[1].z, tc[1].w,
+                                 tc[2].x, tc[2].y, tc[2].z, tc[2].w, tc[3].x, tc[3].y, tc[3].z, tc[3].w};
+#pragma unroll
+            for (int a = 0; a < CV_NN; ++a)
+#pragma unroll
+              for (int r = 0; r < RPT; ++r) acc[r][a] = fmaf(w[r][(m + a) % CV_NN], t[a], acc[r][a]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tc[q] = tn[q];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) w[r][m] = wn[r];
+          }
         }
       }
     }
@@ -203,8 +256,8 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
     if (j >= nJ) continue;
     float* o = A.out + slice * (int64_t)A.W * A.H + (int64_t)(b + CV_NN * j) * A.W;
 #pragma unroll
-    for (int a = 0; a < CV_NN; ++a)
-      if (x_seg + a < A.W) o[x_seg + a] = acc[r][a];
+    for (int a = 0; a < SEG; ++a)
+      if (a < na && x_seg + a < A.W) o[x_seg + a] = acc[r][a];
   }
 }
 
@@ -308,74 +361,80 @@ int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const f
   a.n = n;
   a.kw = (int)kw;
   a.hk = (int)(kw / 2);
-  a.kwp = (a.kw + CV_NN - 1) / CV_NN * CV_NN;
   a.Wv = (kw % 2 == 0) ? a.W - 1 : a.W;  // even kw: the reference's clip never reaches the last column / row
   a.Hv = (kw % 2 == 0) ? a.H - 1 : a.H;
   const int nI = (a.W + CV_NN - 1) / CV_NN, nJ = (a.H + CV_NN - 1) / CV_NN;
   a.tilesX = (nI + 31) / 32;  // at most 32 segments of a row per group, evenly
   a.SX = (nI + a.tilesX - 1) / a.tilesX;
-  a.width = CV_NN * a.SX + a.kwp - 1;
-  a.pitch = a.width;
   auto lanes_of = [&](int rpt) { return n * ((nJ + rpt - 1) / rpt) * (int64_t)a.tilesX * a.SX; };
   const size_t budget = (size_t)optin - 12 * 1024;  // the row table is static
   int smem_sm = 0;
   MLF_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-  // shared memory and group geometry of CTAs of `warps` warps and rpt rows per thread
-  auto plan = [&](int rpt, int warps, ConvArgs& c) {
-    c.gstride = rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
-    while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
-    c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (lanes_of(rpt) + c.SX - 1) / c.SX);
-    const size_t bytes = sizeof(float) * (2 * 16 * (size_t)c.kwp + 2 * (size_t)c.max_groups * c.gstride);
-    return bytes <= budget && c.max_groups * rpt <= CV_MAX_ROWS ? bytes : (size_t)0;
+  // Rows per thread, whole or half segments, and warps per CTA: those with the fewest cycles per
+  // kernel column.  A step takes `lone` cycles while the SM has at most one warp per scheduler, and
+  // `each` cycles of the SM per warp beyond that (measured).  One row of half a segment where that
+  // leaves few warps on an SM (253 x 198 x 4, kw 136: 483 us against 830 with two rows of a whole
+  // segment, 571 with one; 300 x 300 x 30, kw 40: 498 against 414), two rows of a whole segment where
+  // the SMs are full (376 x 376 x 20, kw 241: 9.6 ms against 13.7), and the CTA size that leaves the
+  // shortest last wave.  Two rows of half a segment lose to one or the other everywhere (400 x 400 x 1,
+  // kw 200: 904 us against 884; 376 x 376 x 20: 11.0 ms).
+  struct Variant {
+    int rpt, halves, regs;
+    double lone, each;
+    const void* kernel;
   };
-  // Rows per thread and warps per CTA: the pair with the fewest cycles per kernel column.  A step
-  // takes 60 (one row) or 84 cycles (two rows) while the SM has at most one warp per scheduler, and
-  // 12.2 or 14.5 cycles of the SM per warp beyond that (measured; four rows took 138 and 27, no
-  // better per row).  So one row for a few segments per SM (253 x 198 x 4, kw 136: 0.60 ms against
-  // 0.83 with two), two where the SMs are full (376 x 376 x 77, kw 241: 34 ms against 48), and the
-  // CTA size that leaves the shortest last wave.
-  int rpt = 0, warps = 0;
+  const Variant variants[] = {{1, 2, 80, 26, 5.7, (const void*)k_conv_vec_lanes<1, CV_HALF>},
+                              {2, 1, 112, 84, 14.5, (const void*)k_conv_vec_lanes<2, CV_NN>}};
+  // shared memory and group geometry of CTAs of `warps` warps
+  auto plan = [&](const Variant& v, int warps, ConvArgs& c) {
+    c.kwp = v.halves == 2 ? c.kw : (c.kw + CV_NN - 1) / CV_NN * CV_NN;
+    c.width = c.pitch = CV_NN * c.SX + c.kwp - 1;
+    c.gstride = v.rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
+    while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
+    c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (lanes_of(v.rpt) + c.SX - 1) / c.SX);
+    // half segments read a few floats past their rows and taps
+    const size_t over = v.halves == 2 ? 64 : 0;
+    const size_t bytes = sizeof(float) * (2 * (v.halves == 2 ? CV_HALF : 16) * (size_t)c.kwp +
+                                          2 * (size_t)c.max_groups * c.gstride + over);
+    return bytes <= budget && c.max_groups * v.rpt <= CV_MAX_ROWS ? bytes : (size_t)0;
+  };
+  const Variant* use = nullptr;
+  int warps = 0;
   size_t smem = 0;
   double best = 0;
-  for (int r : {1, 2}) {
-    const double lone = r == 1 ? 60 : 84, each = r == 1 ? 12.2 : 14.5;
-    const int regs = r == 1 ? 80 : 112;
-    const int64_t wp = (lanes_of(r) + 31) / 32;  // warps per phase
+  for (const Variant& v : variants) {
+    const int64_t wp = (lanes_of(v.rpt) + 31) / 32;  // warps per phase (and half)
     for (int k = 1; k <= CV_MAX_THREADS / 32; ++k) {
       ConvArgs c = a;
-      const size_t bytes = plan(r, k, c);
+      const size_t bytes = plan(v, k, c);
       if (!bytes) continue;
-      const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (regs * 32 * k)));
-      const int64_t ctas = CV_NN * ((wp + k - 1) / k);
+      const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (v.regs * 32 * k)));
+      const int64_t ctas = CV_NN * v.halves * ((wp + k - 1) / k);
       const int64_t waves = (ctas + nsm * per_sm - 1) / (nsm * per_sm);
       const int64_t on_sm = std::min<int64_t>(per_sm, (ctas + nsm - 1) / nsm);
       // the busiest of four schedulers; each CTA stages taps and rows of its own, shared by its
-      // warps (idle ones too: 40 x 35 x 2, kw 21 has 18 lanes per phase and takes 90 us with two
-      // warps, 75 with six), whose barriers cost more the more there are
+      // warps (idle ones too: 40 x 35 x 2, kw 21 has 18 lanes per phase and takes 48 us with two
+      // warps, 38 with six), whose barriers cost more the more there are
       const int64_t w = k * on_sm <= 4 ? 4 : (k * on_sm + 3) / 4 * 4;
-      const double stage = 8.0 * (0.5 + (double)(c.max_groups * r) * c.width / (32.0 * a.kw)) / k;
-      const double cyc = (double)waves * (std::max(lone, each * (double)w) + (stage + 2.0) * (double)on_sm + 0.7 * k);
-      if (!rpt || cyc < best) {
+      const double stage = 8.0 * (0.5 / v.halves + (double)(c.max_groups * v.rpt) * c.width / (32.0 * a.kw)) / k;
+      const double cyc = (double)waves * (std::max(v.lone, v.each * (double)w) + (stage + 2.0) * (double)on_sm + 0.35 * k);
+      if (!use || cyc < best) {
         best = cyc;
-        rpt = r;
+        use = &v;
         warps = k;
         smem = bytes;
       }
     }
   }
-  if (!rpt) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
-  plan(rpt, warps, a);
+  if (!use) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
+  plan(*use, warps, a);
   const int threads = 32 * warps;
-  const int64_t lanes = lanes_of(rpt);
+  const int64_t lanes = lanes_of(use->rpt);
   const int64_t ctas = (lanes + threads - 1) / threads;
   if (ctas > INT32_MAX) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: too many slices");
-  const void* kf = rpt == 1 ? (const void*)k_conv_vec_lanes<1> : (const void*)k_conv_vec_lanes<2>;
-  MLF_TRY(allow_max_dyn_smem(kf));
-  const dim3 grid((unsigned)ctas, CV_NN);
-  if (rpt == 1)
-    k_conv_vec_lanes<1><<<grid, threads, smem, st>>>(a);
-  else
-    k_conv_vec_lanes<2><<<grid, threads, smem, st>>>(a);
+  MLF_TRY(allow_max_dyn_smem(use->kernel));
+  void* args[] = {&a};
+  MLF_CUDA(cudaLaunchKernel(use->kernel, dim3((unsigned)ctas, CV_NN * use->halves), dim3(threads), args, smem, st));
   MLF_LAUNCHED();
   return MLF_OK;
 }
