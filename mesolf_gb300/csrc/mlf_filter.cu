@@ -35,10 +35,11 @@ struct FGeo {
   int Z;
 };
 
-// FP64 runs at one operation per SM and cycle or less here, conversions included, so the two uses that
+// FP64 runs at two operations per SM and cycle here, conversions no faster, so the two uses that
 // touch every voxel are kept off it: sums are pairs of floats (each addition's rounding error, exact by
 // TwoSum, goes to the second one; about 48 bits, then FP64 across threads), and the scaling multiplies
-// by a pair, rounding the product once.  45 x 70 x 51 lenslets: row pass 437 -> 350 us, column pass 435 -> 367, k_rephase 205 -> 74.
+// by a pair, rounding the product once.  45 x 70 x 51 lenslets: row pass 437 -> 350 us, column pass
+// 435 -> 367, k_rephase 205 -> 74.
 struct PairSum {
   float s = 0.f, e = 0.f;
   __device__ __forceinline__ void add(float v) {
