@@ -644,7 +644,7 @@ int mlf_batch_plan_bytes(const mlf_psf* psf, int32_t npatch, const int64_t* Xr, 
     li.push_back((int)(Xr[k] / psf->N));
     lj.push_back((int)(Xc[k] / psf->N));
     // filter scratch volume, reduction scratch, filter kernels and sums (upper bounds)
-    const int64_t gmax = (std::max(Xr[k], Xc[k]) + 31) / 32;
+    const int64_t gmax = (std::max(Xr[k], Xc[k]) + kFilterLines - 1) / kFilterLines;
     members += (size_t)(filter_pitch(Xr[k]) * Xc[k] * nz[k] * 4 + 4096 * 8 + (int64_t)nz[k] * (Xr[k] + Xc[k]) * 4 +
                         6 * (int64_t)nz[k] * 4 + (2 * (int64_t)nz[k] * gmax + nz[k]) * 8);
   }

@@ -22,10 +22,13 @@ namespace mlf {
 
 namespace {
 
-constexpr int kLines = 32;      // lines per CTA (one per lane)
-constexpr int kPad = 33;        // shared-memory row stride (bank-conflict free)
+// 16 lines per CTA, a half warp's lanes: their 46 KB at 675 px leave an SM four CTAs that load, filter
+// and store in turn; 32 lines left it one or two: 350 -> 325 us (row pass) and 367 -> 288 (column pass) at
+// 45 x 70 x 51.
+constexpr int kLines = kFilterLines;
+constexpr int kPad = 17;        // shared-memory row stride (bank-conflict free)
 constexpr int kChunk = 8;       // consecutive outputs per thread
-constexpr int kFiltThreads = 512;
+constexpr int kFiltThreads = 256;
 constexpr int kLoadUnroll = 8;   // loads in flight per thread while staging lines
 
 // The filter's scratch V: MATLAB layout with lines Vp = filter_pitch(Xr) floats apart, a multiple of 4,
@@ -83,7 +86,7 @@ __global__ void k_rephase(const float* __restrict__ V, FGeo f, const double* __r
 // buf[i * kPad + line].  taps[k] = c[(k - wlo) mod L] for k < nt, zero for nt <= k < ntp
 // (ntp a multiple of 8, taps in shared memory, 16-byte aligned):
 //   y[i] = sum_k taps[k] * x[(i + wlo - k) mod L]
-// Each thread produces kChunk = 8 consecutive outputs of one line (lane = line) and walks the
+// Each thread produces kChunk = 8 consecutive outputs of one line (a half warp's lanes: the lines) and walks the
 // taps in groups of 8 over a 16-value register window, so one group costs 8 window loads
 // and 2 tap loads for 64 FMAs.  Every output adds its products in the order k = 0, 1, ...
 // (the zero taps add exactly nothing).
@@ -92,11 +95,13 @@ template <class Emit>
 __device__ double filter_lines(const float* __restrict__ buf, int L, const float* __restrict__ taps,
                                int ntp, int wlo, int nlines, Emit emit) {
   static_assert(kChunk == 8, "the register window assumes 8 outputs per thread");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x % kLines, half = threadIdx.x % 32 / kLines, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   PairSum s;
   const int nchunks = (L + kChunk - 1) / kChunk;
-  for (int chk = warp; chk < nchunks; chk += nwarps) {
-    if (lane >= nlines) continue;
+  // a warp's halves take chunks two apart: 16 rows of 17 floats put them on different banks
+  for (int p = warp; 4 * (p / 2) + p % 2 < nchunks; p += nwarps) {
+    const int chk = 4 * (p / 2) + p % 2 + 2 * half;
+    if (lane >= nlines || chk >= nchunks) continue;
     const int i0 = chk * kChunk;
     const int j = (i0 + wlo) % L;  // index of x for output i0 at k = 0
     float w[16];                    // w[m] = x[(j - k0 - 8 + m) mod L] within the group at k0
@@ -203,18 +208,18 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
   const int ntp = stage_taps(tsm, cy + (int64_t)e * tap_stride, nt_e[e]);
   const int nlines = (int)(g.Xr - r0 < kLines ? g.Xr - r0 : kLines);
   float* plane = V + (int64_t)z * g.Vp * g.Xc;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x % kLines, col = threadIdx.x / kLines, ncols = blockDim.x / kLines;
   // 8 column loads in flight per thread
-  for (int c0 = warp; c0 < (int)g.Xc; c0 += kLoadUnroll * nwarps) {
+  for (int c0 = col; c0 < (int)g.Xc; c0 += kLoadUnroll * ncols) {
     float v[kLoadUnroll];
 #pragma unroll
     for (int u = 0; u < kLoadUnroll; ++u) {
-      const int c = c0 + u * nwarps;
+      const int c = c0 + u * ncols;
       v[u] = (c < g.Xc && lane < nlines) ? plane[(int64_t)c * g.Vp + r0 + lane] : 0.f;
     }
 #pragma unroll
     for (int u = 0; u < kLoadUnroll; ++u) {
-      const int c = c0 + u * nwarps;
+      const int c = c0 + u * ncols;
       if (c < g.Xc && lane < nlines) buf[c * kPad + lane] = v[u];
     }
   }
@@ -228,21 +233,28 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
   block_reduce_store(s, sums_out + (int64_t)blockIdx.y * gridDim.x + blockIdx.x);
 }
 
-// scale[z] = sum_before / sum_after for filtered planes (fixed-order sums), 1 otherwise.
+// scale[z] = sum_before / sum_after for filtered planes (fixed-order sums, one warp per plane), 1
+// otherwise.
 __global__ void k_filter_scale(const double* sin, int nin, const double* sout, int nout,
                                const int* zlist, int nzf, int Z, double* scale) {
-  const int z = blockIdx.x * blockDim.x + threadIdx.x;
-  if (z >= Z) return;
+  const int z = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (z >= Z) return;  // whole warps
   int k = -1;
-  for (int t = 0; t < nzf; ++t)
+  for (int t = lane; t < nzf; t += 32)
     if (zlist[t] == z) k = t;
+  k = __reduce_max_sync(0xffffffffu, k);
   if (k < 0) {
-    scale[z] = 1.0;
+    if (lane == 0) scale[z] = 1.0;
     return;
   }
   double a = 0.0, b = 0.0;
-  for (int i = 0; i < nin; ++i) a += sin[(int64_t)k * nin + i];
-  for (int i = 0; i < nout; ++i) b += sout[(int64_t)k * nout + i];
+  for (int i = lane; i < nin; i += 32) a += sin[(int64_t)k * nin + i];
+  for (int i = lane; i < nout; i += 32) b += sout[(int64_t)k * nout + i];
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane != 0) return;
   // An all-zero plane (flux underflowed to 0) stays zero.  The reference's
   // sum_before * buf / sum(buf) would give 0/0 = NaN there (…_with_filter.m:233), which the
   // next update's blend (1-w)*X would carry forward; FP32 planes reach exact zero long
@@ -393,7 +405,9 @@ int filter_init(Solver* s) {
   const size_t smem_c = sizeof(float) * ((size_t)taps_offset(Lc) + ((Lc + 7) & ~7));
   int dev_smem = 0;
   MLF_CUDA(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-  if ((int)std::max(smem_r, smem_c) > dev_smem)
+  // sides whose 32-line buffers did not fit were refused and still are
+  const int side = std::max(Lr, Lc);
+  if ((int)std::max(smem_r, smem_c) > dev_smem || (int)sizeof(float) * (((side * 33 + 3) & ~3) + ((side + 7) & ~7)) > dev_smem)
     return fail(MLF_ERR_UNSUPPORTED, "image side too large for the sample filter's line buffers");
   MLF_TRY(allow_max_dyn_smem((const void*)k_filter_r));
   MLF_TRY(allow_max_dyn_smem((const void*)k_filter_c));
@@ -426,7 +440,7 @@ int filter_run_geo(Solver* s, const PatchGeo& g, float* X, cudaStream_t st) {
       X, g, V, fg, zl, pe, f.cx.as<float>(), wlo_x, nt_x, Lr, sin);
   k_filter_c<<<dim3(gc, nzf), kFiltThreads, sizeof(float) * ((size_t)taps_offset(Lc) + ((Lc + 7) & ~7)), st>>>(
       V, fg, zl, pe, f.cy.as<float>(), wlo_y, nt_y, Lc, sout);
-  k_filter_scale<<<(Z + 255) / 256, 256, 0, st>>>(sin, gr, sout, gc, zl, nzf, Z, scale);
+  k_filter_scale<<<(Z + 7) / 8, 256, 0, st>>>(sin, gr, sout, gc, zl, nzf, Z, scale);
   k_rephase<<<dim3((Lc + kPhaseLines - 1) / kPhaseLines, nzf), 256,
               sizeof(float) * (phase_tab_floats(g.N) + kPhaseLines * Lr), st>>>(
       V, fg, scale, zl, g, X);

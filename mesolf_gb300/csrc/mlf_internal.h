@@ -220,6 +220,7 @@ int rl_view_step(Solver* s, const float* d_lf, float* d_vol, int u, int v, doubl
 int launch_extract_views(const float* d_lf, const PatchGeo& g, float* lfs, int64_t view_stride, int64_t off,
                          cudaStream_t st);
 // line pitch (floats) of the filter's scratch volume; at most N * Pa, the volume's own
+constexpr int kFilterLines = 16;  // lines per CTA of the filter's passes: their sums' blocks
 inline int64_t filter_pitch(int64_t Xr) { return (Xr + 3) / 4 * 4; }
 int launch_to_phase(const float* d_vol, const PatchGeo& g, float* X, cudaStream_t st,
                     const float* zscale = nullptr);
