@@ -136,16 +136,23 @@ k_si_tnorm(const float* __restrict__ t_part, int ps, int64_t T, const float* __r
   __shared__ float shf[32];
   const int tid = threadIdx.x;
   for (int64_t j = tid; j < T; j += SI_RED_THREADS) {
-    float v = 0.f;
-    for (int s0 = 0; s0 < ps; s0 += 16) {  // 16 splits' loads in flight, added in order
+    // 16 splits' loads in flight, added pairwise; their sums with compensation (up to 152 splits: one
+    // chain of additions put 2.3e-7 into t at 165 x 165 x 140, where a few long splits had 7e-8)
+    float v = 0.f, l = 0.f;
+    for (int s0 = 0; s0 < ps; s0 += 16) {
       float x[16];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) x[u] = t_part[(int64_t)min(s0 + u, ps - 1) * T + j];
+      for (int u = 0; u < 16; ++u) x[u] = s0 + u < ps ? t_part[(int64_t)(s0 + u) * T + j] : 0.f;
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
-        if (s0 + u < ps) v += x[u];
+      for (int st = 8; st > 0; st >>= 1)
+#pragma unroll
+        for (int u = 0; u < st; ++u) x[u] += x[u + st];
+      float s, e;
+      two_sum(v, x[0], s, e);
+      v = s;
+      l += e;
     }
-    t[j] = v;
+    t[j] = v + l;
   }
   __syncthreads();
   if (tid < NS) {
