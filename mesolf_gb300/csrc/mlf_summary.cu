@@ -40,8 +40,8 @@ constexpr int SI_ROW_U = 8;         // float4 frames prefetched per plain row-pa
 constexpr int SI_PIX_U = 32;        // frames prefetched per pixelwise group
 constexpr int SI_RED_THREADS = 1024;
 
-// scal[]: 0 M, 1 1/M, 2 mean(t), 3 max(img)
-enum { SC_M = 0, SC_INVM = 1, SC_TMEAN = 2, SC_IMGMAX = 3, SC_N = 4 };
+// scal[]: 0 M, 1 1/M, 2 max(img)
+enum { SC_M = 0, SC_INVM = 1, SC_IMGMAX = 2, SC_N = 3 };
 
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   s = a + b;
@@ -123,16 +123,16 @@ k_si_coldot(const float* __restrict__ Y, int64_t P, int64_t T, const float* __re
   }
 }
 
-// One block: t = sum over splits of t_part (fixed order), t /= |t| (FP64 norm), mean(t);
+// One block: t = sum over splits of t_part (fixed order), t /= |t| (FP64 norm);
 // nmax > 0: M = max(max_part[0..nmax)).
 // Bound: latency of the one block, and FP64, of which an SM does two operations a cycle: so four
-// warps take the two FP64 sums (32 warps' shuffles alone cost 2 x 1.3 us) and the division by the
+// warps take the FP64 sum (32 warps' shuffles alone cost 2 x 1.3 us) and the division by the
 // norm is one reciprocal.
 __global__ void __launch_bounds__(SI_RED_THREADS)
 k_si_tnorm(const float* __restrict__ t_part, int ps, int64_t T, const float* __restrict__ max_part, int64_t nmax,
            float* __restrict__ t, float* __restrict__ scal) {
-  constexpr int NS = 128;  // threads of the FP64 sums
-  __shared__ double shd[2][NS / 32];
+  constexpr int NS = 128;  // threads of the FP64 sum
+  __shared__ double shd[NS / 32];
   __shared__ float shf[32];
   const int tid = threadIdx.x;
   for (int64_t j = tid; j < T; j += SI_RED_THREADS) {
@@ -156,28 +156,20 @@ k_si_tnorm(const float* __restrict__ t_part, int ps, int64_t T, const float* __r
   }
   __syncthreads();
   if (tid < NS) {
-    double ss = 0.0, st = 0.0;
+    double ss = 0.0;
     for (int64_t j = tid; j < T; j += NS) {
       const double v = t[j];
       ss += v * v;
-      st += v;
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      ss += __shfl_down_sync(0xffffffffu, ss, o);
-      st += __shfl_down_sync(0xffffffffu, st, o);
-    }
-    if ((tid & 31) == 0) {
-      shd[0][tid >> 5] = ss;
-      shd[1][tid >> 5] = st;
-    }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) shd[tid >> 5] = ss;
   }
   __shared__ double rn;
   __syncthreads();
-  if (tid == 0) rn = 1.0 / sqrt((shd[0][0] + shd[0][1]) + (shd[0][2] + shd[0][3]));
+  if (tid == 0) rn = 1.0 / sqrt((shd[0] + shd[1]) + (shd[2] + shd[3]));
   __syncthreads();
   const double rnrm = rn;
   for (int64_t j = tid; j < T; j += SI_RED_THREADS) t[j] = (float)((double)t[j] * rnrm);
-  if (tid == 0) scal[SC_TMEAN] = (float)(((shd[1][0] + shd[1][1]) + (shd[1][2] + shd[1][3])) * rnrm / (double)T);
   if (nmax > 0) {
     float m = -INFINITY;
     for (int64_t i = tid; i < nmax; i += SI_RED_THREADS) m = fmaxf(m, max_part[i]);
@@ -591,12 +583,30 @@ k_si_pixelwise(const float* __restrict__ Y, int64_t P, int T, const float* __res
 // Last pass, 'global': s and compute_std_image(Y/M, s, t) as written in the reference.  The
 // expansion cancels terms of the size of mean(y)^2 against each other, so sum(y^2), sum(y)
 // and s carry TwoSum compensation (s also the exact product error) and the formula runs in
-// FP64 per pixel.
+// FP64 per pixel.  There s and mean(t) are divided by the norm of the FP32 t, which its rounding leaves
+// 2^-25 / sqrt(T) off one: s^2 / T is a thousand times the variance left, so that error alone put up to
+// 3e-6 into the image at 140 frames.
 __global__ void __launch_bounds__(SI_ROW_THREADS)
 k_si_global(const float* __restrict__ Y, int64_t P, int64_t T, const float* __restrict__ t,
             const float* __restrict__ scal, float* __restrict__ s_out, float* __restrict__ img,
             float* __restrict__ img_max_part) {
   __shared__ float sh[32];
+  __shared__ double shd[32], tn[2];
+  {
+    double n2 = 0.0, m = 0.0;
+    for (int64_t j = threadIdx.x; j < T; j += SI_ROW_THREADS) {
+      const double v = __ldg(t + j);
+      n2 += v * v;
+      m += v;
+    }
+    n2 = block_sum(n2, shd);
+    m = block_sum(m, shd);
+    if (threadIdx.x == 0) {
+      tn[0] = 1.0 / sqrt(n2);
+      tn[1] = m / (double)T;
+    }
+    __syncthreads();
+  }
   const int64_t p = (int64_t)blockIdx.x * SI_ROW_THREADS + threadIdx.x;
   float v_img = -INFINITY;
   if (p < P) {
@@ -631,9 +641,9 @@ k_si_global(const float* __restrict__ Y, int64_t P, int64_t T, const float* __re
     for (; j < T; ++j) acc(__ldcs(y + j * P), __ldg(t + j));
     const double sd = (double)S + (double)LS;  // Y/M already applied: s = (Y/M) t
     s_out[p] = (float)sd;
-    const double Tn = (double)T, C = (double)scal[SC_TMEAN];
+    const double Tn = (double)T, su = sd * tn[0], C = tn[1] * tn[0];  // of the unit t
     const double Ad = (double)A + (double)LA, Bm = ((double)B + (double)LB) / Tn;
-    const double v = (Ad - sd * sd) / Tn - Bm * Bm + 2.0 * Bm * sd * C - sd * sd * C * C;
+    const double v = (Ad - su * su) / Tn - Bm * Bm + 2.0 * Bm * su * C - su * su * C * C;
     v_img = (float)sqrt(fmax(v, 0.0));
     img[p] = v_img;
   }
