@@ -95,6 +95,13 @@ int mlf_probe_fp32_peak(double ms, double* tflops, void* stream);
  * reference. */
 int mlf_probe_wait_timeout(uint32_t limit, void* stream);
 
+/* Test support: the FP32 view kernel's launch shape of a solver.  plan[0], plan[1]: tile rows and
+ * columns, plan[2]: channel slots per CTA, plan[3]: CTAs, plan[4]: partial planes that the reduction
+ * adds.  With poison != 0 every value of the forward partials becomes NaN (on `stream`), so that a
+ * plane which is read without having been written shows in the results.  No counterpart in the
+ * reference. */
+int mlf_probe_view_plan(mlf_solver* s, int64_t plan[5], int32_t poison, void* stream);
+
 /* Copy the calling thread's last error message into buf (always NUL-terminated).
  * Returns the status code of that error. */
 int mlf_last_error(char* buf, size_t len);

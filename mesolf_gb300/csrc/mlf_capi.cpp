@@ -571,6 +571,19 @@ int mlf_solver_destroy(mlf_solver* s) {
 
 int64_t mlf_solver_device_bytes(const mlf_solver* s) { return s ? (int64_t)s->bytes() : 0; }
 
+int mlf_probe_view_plan(mlf_solver* s, int64_t plan[5], int32_t poison, void* stream) {
+  clear_error();
+  if (!s || !plan) return fail(MLF_ERR_INVALID, "mlf_probe_view_plan: null pointer");
+  plan[0] = s->tileY;
+  plan[1] = s->tileX;
+  plan[2] = s->slots;
+  plan[3] = s->grid;
+  plan[4] = view_partials(s);
+  // all bits set: a NaN
+  if (poison) MLF_CUDA(cudaMemsetAsync(s->part.p, 0xff, s->part.bytes, static_cast<cudaStream_t>(stream)));
+  return MLF_OK;
+}
+
 int mlf_solver_run(mlf_solver* s, const float* lfimg, int32_t max_iter, int32_t precision,
                    const float* warm_start, float* vol_out, mlf_stats* stats, void* stream) {
   mlf::Range nvtx_range("mlf_solver_run");

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <string>
@@ -366,6 +367,11 @@ constexpr int VWS_TX = 4;
 constexpr int kViewMaxThreads = 320;
 // Whether a CTA adds its slots' forward partials itself (the comment at the sum in k_view).
 __host__ __device__ constexpr bool view_sums_slots(int slots) { return slots > 2; }
+// Partial planes that the reduction adds: one per CTA, or one per slot.  Plane blockIdx * slots + slot is
+// written when it has a channel, so with an odd channel count the second slot of the last CTA has none.
+inline int64_t view_partials(const Solver* s) {
+  return view_sums_slots(s->slots) ? s->grid : std::min((int64_t)s->grid * s->slots, s->nch);
+}
 // Staged planes of the view kernel (ratio image, forward input) are stored with their
 // 16-byte column chunks swizzled: in every other 32-float block the chunks of each pair
 // trade places (column c lives at c ^ 4 when bit 5 of c is set), except a last chunk whose

@@ -442,7 +442,7 @@ int run_reduce(Solver* s, int view, float* hx_out, bool ratio, cudaStream_t st) 
   const int HP = s->tilesA * s->tileX;
   const int group = view_sums_slots(s->slots) ? s->slots : 1;  // planes that the view kernel has added
   const float* part = s->part.as<float>();
-  int nparts = s->grid * s->slots / group, Li = s->Li, Lj = s->Lj, hp = HP, RP = s->RP, off = s->q + 1;
+  int nparts = (int)view_partials(s), Li = s->Li, Lj = s->Lj, hp = HP, RP = s->RP, off = s->q + 1;
   int64_t ppl = (int64_t)group * s->tilesB * s->tileY * HP;
   float* rpad = ratio ? s->rpad.as<float>() : nullptr;
   void* args[] = {&part, &nparts, &Li, &Lj, &hp, &ppl, &lfsub, &hx_out, &rpad, &RP, &off};
