@@ -252,13 +252,17 @@ __global__ void k_scatter_views(const float* __restrict__ lfs, PatchGeo g, float
 // kReduceGroups, ... and their sums are added in a fixed order (deterministic).  Bound by the
 // latency of the L2 reads, so 32 warps share the planes (31 x 40 lenslets: 22.6 us for 1824
 // slot planes on 8 warps, 4.2 us for the 456 planes that the CTAs leave on 32).
+// The next view kernel may be launched once the sums are formed, so that its CTAs settle on SMs that the
+// view kernel before has left.  With the launch at this kernel's start they were placed while that one
+// still ran, and patches of middle size took up to half again as long (one iteration of 60 x 60 x 25
+// lenslets, T 11: 42.6 -> 28.4 ms, of 58 x 58 x 51, T 15: 143 -> 126, without dependent launches 28.8
+// and 126; four of 11 x 11 x 21, T 3: 5.35 -> 5.04, without 6.99).
 constexpr int kReduceGroups = 32;
 __global__ void __launch_bounds__(32 * kReduceGroups)
 k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int HP, int64_t PPL,
                const float* __restrict__ lfsub, float* __restrict__ hx_out,
                float* __restrict__ rpad, int RP, int off) {
   __shared__ float sh[kReduceGroups][32];
-  pdl_launch_dependents();
   pdl_wait();
   const int LL = Li * Lj;
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
@@ -281,6 +285,7 @@ k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int H
   }
   sh[grp][lane] = s;
   __syncthreads();
+  pdl_launch_dependents();
   if (grp != 0 || i >= LL) return;
   float t[kReduceGroups];  // pairwise: a short chain, and a rounding error that does not grow with it
 #pragma unroll
