@@ -259,7 +259,7 @@ __global__ void k_scatter_views(const float* __restrict__ lfs, PatchGeo g, float
 // and 126; four of 11 x 11 x 21, T 3: 5.35 -> 5.04, without 6.99).
 constexpr int kReduceGroups = 32;
 __global__ void __launch_bounds__(32 * kReduceGroups)
-k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int HP, int64_t PPL,
+k_reduce_ratio(const float* part, int nparts, int Li, int Lj, int HP, int64_t PPL,
                const float* __restrict__ lfsub, float* __restrict__ hx_out,
                float* __restrict__ rpad, int RP, int off) {
   __shared__ float sh[kReduceGroups][32];
@@ -270,17 +270,18 @@ k_reduce_ratio(const float* __restrict__ part, int nparts, int Li, int Lj, int H
   const int a = i % Li, b = i / Li;
   const float* pp = part + (int64_t)b * HP + a;
   float s = 0.f;
+  // the view kernel may write `part` during this kernel's life, until pdl_wait: no read-only loads
   if (i < LL) {
     float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
     int k = grp;
 #pragma unroll 3
     for (; k + 3 * kReduceGroups < nparts; k += 4 * kReduceGroups) {
-      s0 += pp[k * PPL];
-      s1 += pp[(k + kReduceGroups) * PPL];
-      s2 += pp[(k + 2 * kReduceGroups) * PPL];
-      s3 += pp[(k + 3 * kReduceGroups) * PPL];
+      s0 += __ldcg(pp + k * PPL);
+      s1 += __ldcg(pp + (k + kReduceGroups) * PPL);
+      s2 += __ldcg(pp + (k + 2 * kReduceGroups) * PPL);
+      s3 += __ldcg(pp + (k + 3 * kReduceGroups) * PPL);
     }
-    for (; k < nparts; k += kReduceGroups) s0 += pp[k * PPL];
+    for (; k < nparts; k += kReduceGroups) s0 += __ldcg(pp + k * PPL);
     s = (s0 + s1) + (s2 + s3);
   }
   sh[grp][lane] = s;
