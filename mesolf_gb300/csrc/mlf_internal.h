@@ -297,8 +297,8 @@ int launch_mex_crop(const float* src, int64_t Wp, int64_t Hq, int64_t W, int64_t
 
 // Programmatic dependent launch: a kernel launched with launch_pdl may start before the kernel
 // before it in the stream has ended, and calls pdl_wait before it reads or overwrites anything that
-// kernel, or one before it, writes or reads.  Every launch_pdl kernel calls pdl_wait in all its
-// threads, so that the order of a chain of them is kept.
+// kernel, or one before it, writes or reads (but the stop words: see k_view).  Every launch_pdl kernel
+// calls pdl_wait in all its threads, so that the order of a chain of them is kept.
 cudaError_t launch_pdl(const void* f, int grid, int threads, void** args, size_t smem, cudaStream_t st);
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -245,7 +245,10 @@ __global__ void __launch_bounds__(kViewMaxThreads, 2) k_view(ViewArgs A) {
   for (int k = 0; k < NC; ++k) xc[k] = view_pcol(a0 + QP + 4 * k, A.XP);
 
   // ---- a cancelled solve: the rest of its view steps return at once (CTA-uniform, at the first
-  // barrier; until then nothing but shared memory is written)
+  // barrier; until then nothing but shared memory and the stop words is written).  Read before
+  // pdl_wait, beside the loads below: the kernel that launched this one early, the reduction, does so
+  // after its own wait, when the view kernel before has ended, so no view step is left half done by a
+  // stop word that the next one sets.
   __shared__ int s_stop;
   if (tid == 0) s_stop = cancel_entry(A.cancel);
 
