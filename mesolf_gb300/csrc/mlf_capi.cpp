@@ -571,6 +571,14 @@ int mlf_solver_destroy(mlf_solver* s) {
 
 int64_t mlf_solver_device_bytes(const mlf_solver* s) { return s ? (int64_t)s->bytes() : 0; }
 
+int mlf_probe_conv_plan(int64_t W, int64_t H, int64_t n, int64_t kw, int32_t sms, int32_t smem_cta, int32_t smem_sm,
+                        int32_t variant, int64_t plan[9]) {
+  clear_error();
+  if (!plan || W < 1 || H < 1 || n < 1 || kw < 1 || sms < 1)
+    return fail(MLF_ERR_INVALID, "mlf_probe_conv_plan: empty call or null pointer");
+  return conv_plan_probe(W, H, n, kw, sms, smem_cta, smem_sm, variant, plan);
+}
+
 int mlf_probe_view_plan(mlf_solver* s, int64_t plan[5], int32_t poison, void* stream) {
   clear_error();
   if (!s || !plan) return fail(MLF_ERR_INVALID, "mlf_probe_view_plan: null pointer");

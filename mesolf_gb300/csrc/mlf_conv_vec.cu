@@ -343,19 +343,23 @@ int launch_mex_crop(const float* src, int64_t Wp, int64_t Hq, int64_t W, int64_t
   return MLF_OK;
 }
 
-int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const float* d_kernels,
-                 int64_t kw, int nnum, float* d_out, cudaStream_t st) {
-  if (nnum != CV_NN) return fail(MLF_ERR_INVALID, "direct MEX projector: the kernel grid must be 15 x 15");
-  if (W > (1 << 24) || H > (1 << 24) || W * H > ((int64_t)1 << 31))
-    return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: slice larger than 2^31 pixels");
-  int dev = 0, optin = 0, nsm = 0;
-  MLF_CUDA(cudaGetDevice(&dev));
-  MLF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+namespace {
+
+struct ConvVariant {
+  int rpt, halves, regs;
+  double lone, each;
+  const void* kernel;
+};
+constexpr int CV_VARIANTS = 2;
+const ConvVariant* conv_variants() {
+  static const ConvVariant v[CV_VARIANTS] = {{1, 2, 80, 26, 5.7, (const void*)k_conv_vec_lanes<1, CV_HALF>},
+                                             {2, 1, 112, 84, 14.5, (const void*)k_conv_vec_lanes<2, CV_NN>}};
+  return v;
+}
+
+// The sizes of a call, less its pointers.
+ConvArgs conv_sizes(int64_t W, int64_t H, int64_t n, int64_t kw) {
   ConvArgs a{};
-  a.in = d_bitmap;
-  a.K = d_kernels;
-  a.out = d_out;
   a.W = (int)W;
   a.H = (int)H;
   a.n = n;
@@ -363,50 +367,55 @@ int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const f
   a.hk = (int)(kw / 2);
   a.Wv = (kw % 2 == 0) ? a.W - 1 : a.W;  // even kw: the reference's clip never reaches the last column / row
   a.Hv = (kw % 2 == 0) ? a.H - 1 : a.H;
-  const int nI = (a.W + CV_NN - 1) / CV_NN, nJ = (a.H + CV_NN - 1) / CV_NN;
+  const int nI = (a.W + CV_NN - 1) / CV_NN;
   a.tilesX = (nI + 31) / 32;  // at most 32 segments of a row per group, evenly
   a.SX = (nI + a.tilesX - 1) / a.tilesX;
-  auto lanes_of = [&](int rpt) { return n * ((nJ + rpt - 1) / rpt) * (int64_t)a.tilesX * a.SX; };
-  const size_t budget = (size_t)optin - 12 * 1024;  // the row table is static
-  int smem_sm = 0;
-  MLF_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-  // Rows per thread, whole or half segments, and warps per CTA: those with the fewest cycles per
-  // kernel column.  A step takes `lone` cycles while the SM has at most one warp per scheduler, and
-  // `each` cycles of the SM per warp beyond that (measured).  One row of half a segment where that
-  // leaves few warps on an SM (253 x 198 x 4, kw 136: 483 us against 830 with two rows of a whole
-  // segment, 571 with one; 300 x 300 x 30, kw 40: 498 against 414), two rows of a whole segment where
-  // the SMs are full (376 x 376 x 20, kw 241: 9.6 ms against 13.7), and the CTA size that leaves the
-  // shortest last wave.  Two rows of half a segment lose to one or the other everywhere (400 x 400 x 1,
-  // kw 200: 904 us against 884; 376 x 376 x 20: 11.0 ms).
-  struct Variant {
-    int rpt, halves, regs;
-    double lone, each;
-    const void* kernel;
-  };
-  const Variant variants[] = {{1, 2, 80, 26, 5.7, (const void*)k_conv_vec_lanes<1, CV_HALF>},
-                              {2, 1, 112, 84, 14.5, (const void*)k_conv_vec_lanes<2, CV_NN>}};
-  // shared memory and group geometry of CTAs of `warps` warps
-  auto plan = [&](const Variant& v, int warps, ConvArgs& c) {
-    c.kwp = v.halves == 2 ? c.kw : (c.kw + CV_NN - 1) / CV_NN * CV_NN;
-    c.width = c.pitch = CV_NN * c.SX + c.kwp - 1;
-    c.gstride = v.rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
-    while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
-    c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (lanes_of(v.rpt) + c.SX - 1) / c.SX);
-    // half segments read a few floats past their rows and taps
-    const size_t over = v.halves == 2 ? 64 : 0;
-    const size_t bytes = sizeof(float) * (2 * (v.halves == 2 ? CV_HALF : 16) * (size_t)c.kwp +
-                                          2 * (size_t)c.max_groups * c.gstride + over);
-    return bytes <= budget && c.max_groups * v.rpt <= CV_MAX_ROWS ? bytes : (size_t)0;
-  };
-  const Variant* use = nullptr;
-  int warps = 0;
+  return a;
+}
+int64_t conv_lanes(const ConvArgs& a, int rpt) {
+  const int nJ = (a.H + CV_NN - 1) / CV_NN;
+  return a.n * ((nJ + rpt - 1) / rpt) * (int64_t)a.tilesX * a.SX;
+}
+
+// Shared memory and group geometry of CTAs of `warps` warps; 0: they do not fit.
+size_t conv_fit(const ConvVariant& v, int warps, size_t budget, ConvArgs& c) {
+  c.kwp = v.halves == 2 ? c.kw : (c.kw + CV_NN - 1) / CV_NN * CV_NN;
+  c.width = c.pitch = CV_NN * c.SX + c.kwp - 1;
+  c.gstride = v.rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
+  while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
+  c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (conv_lanes(c, v.rpt) + c.SX - 1) / c.SX);
+  // the rings read ahead, a few floats past their rows and taps: the last row's are past its group
+  // where the stride has no padding
+  constexpr size_t over = 64;
+  const size_t bytes = sizeof(float) * (2 * (v.halves == 2 ? CV_HALF : 16) * (size_t)c.kwp +
+                                        2 * (size_t)c.max_groups * c.gstride + over);
+  return bytes <= budget && c.max_groups * v.rpt <= CV_MAX_ROWS ? bytes : (size_t)0;
+}
+
+struct ConvPlan {
+  int variant = -1, warps = 0;
   size_t smem = 0;
+};
+// Rows per thread, whole or half segments, and warps per CTA: those with the fewest cycles per
+// kernel column.  A step takes `lone` cycles while the SM has at most one warp per scheduler, and
+// `each` cycles of the SM per warp beyond that (measured).  One row of half a segment where that
+// leaves few warps on an SM (253 x 198 x 4, kw 136: 483 us against 830 with two rows of a whole
+// segment, 571 with one; 300 x 300 x 30, kw 40: 498 against 414), two rows of a whole segment where
+// the SMs are full (376 x 376 x 20, kw 241: 9.6 ms against 13.7), and the CTA size that leaves the
+// shortest last wave.  Two rows of half a segment lose to one or the other everywhere (400 x 400 x 1,
+// kw 200: 904 us against 884; 376 x 376 x 20: 11.0 ms).
+// only: that variant alone (-1: any).
+ConvPlan conv_plan(const ConvArgs& a, int nsm, int optin, int smem_sm, int only) {
+  const size_t budget = (size_t)optin - 12 * 1024;  // the row table is static
+  ConvPlan p;
   double best = 0;
-  for (const Variant& v : variants) {
-    const int64_t wp = (lanes_of(v.rpt) + 31) / 32;  // warps per phase (and half)
+  for (int i = 0; i < CV_VARIANTS; ++i) {
+    if (only >= 0 && i != only) continue;
+    const ConvVariant& v = conv_variants()[i];
+    const int64_t wp = (conv_lanes(a, v.rpt) + 31) / 32;  // warps per phase (and half)
     for (int k = 1; k <= CV_MAX_THREADS / 32; ++k) {
       ConvArgs c = a;
-      const size_t bytes = plan(v, k, c);
+      const size_t bytes = conv_fit(v, k, budget, c);
       if (!bytes) continue;
       const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (v.regs * 32 * k)));
       const int64_t ctas = CV_NN * v.halves * ((wp + k - 1) / k);
@@ -418,23 +427,54 @@ int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const f
       const int64_t w = k * on_sm <= 4 ? 4 : (k * on_sm + 3) / 4 * 4;
       const double stage = 8.0 * (0.5 / v.halves + (double)(c.max_groups * v.rpt) * c.width / (32.0 * a.kw)) / k;
       const double cyc = (double)waves * (std::max(v.lone, v.each * (double)w) + (stage + 2.0) * (double)on_sm + 0.35 * k);
-      if (!use || cyc < best) {
+      if (p.variant < 0 || cyc < best) {
         best = cyc;
-        use = &v;
-        warps = k;
-        smem = bytes;
+        p = ConvPlan{i, k, bytes};
       }
     }
   }
-  if (!use) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
-  plan(*use, warps, a);
-  const int threads = 32 * warps;
-  const int64_t lanes = lanes_of(use->rpt);
-  const int64_t ctas = (lanes + threads - 1) / threads;
+  return p;
+}
+
+}  // namespace
+
+int conv_plan_probe(int64_t W, int64_t H, int64_t n, int64_t kw, int nsm, int optin, int smem_sm, int variant,
+                    int64_t out[9]) {
+  ConvArgs a = conv_sizes(W, H, n, kw);
+  const ConvPlan p = conv_plan(a, nsm, optin, smem_sm, variant);
+  if (p.variant < 0) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
+  const ConvVariant& v = conv_variants()[p.variant];
+  conv_fit(v, p.warps, (size_t)optin, a);
+  const int64_t o[9] = {p.variant, p.warps, (int64_t)p.smem, a.kwp, a.SX, a.pitch, a.gstride, a.max_groups,
+                        conv_lanes(a, v.rpt)};
+  std::copy(o, o + 9, out);
+  return MLF_OK;
+}
+
+int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const float* d_kernels,
+                 int64_t kw, int nnum, float* d_out, cudaStream_t st) {
+  if (nnum != CV_NN) return fail(MLF_ERR_INVALID, "direct MEX projector: the kernel grid must be 15 x 15");
+  if (W > (1 << 24) || H > (1 << 24) || W * H > ((int64_t)1 << 31))
+    return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: slice larger than 2^31 pixels");
+  int dev = 0, optin = 0, nsm = 0, smem_sm = 0;
+  MLF_CUDA(cudaGetDevice(&dev));
+  MLF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  MLF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  MLF_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  ConvArgs a = conv_sizes(W, H, n, kw);
+  a.in = d_bitmap;
+  a.K = d_kernels;
+  a.out = d_out;
+  const ConvPlan p = conv_plan(a, nsm, optin, smem_sm, -1);
+  if (p.variant < 0) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
+  const ConvVariant& v = conv_variants()[p.variant];
+  conv_fit(v, p.warps, (size_t)optin, a);
+  const int threads = 32 * p.warps;
+  const int64_t ctas = (conv_lanes(a, v.rpt) + threads - 1) / threads;
   if (ctas > INT32_MAX) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: too many slices");
-  MLF_TRY(allow_max_dyn_smem(use->kernel));
+  MLF_TRY(allow_max_dyn_smem(v.kernel));
   void* args[] = {&a};
-  MLF_CUDA(cudaLaunchKernel(use->kernel, dim3((unsigned)ctas, CV_NN * use->halves), dim3(threads), args, smem, st));
+  MLF_CUDA(cudaLaunchKernel(v.kernel, dim3((unsigned)ctas, CV_NN * v.halves), dim3(threads), args, p.smem, st));
   MLF_LAUNCHED();
   return MLF_OK;
 }
