@@ -99,9 +99,9 @@ int mlf_probe_wait_timeout(uint32_t limit, void* stream);
  * bytes of shared memory per CTA and smem_sm per SM (host arithmetic only).  variant: 0 half segments,
  * 1 whole ones in two rows, -1 the faster one.  plan[0] variant, [1] warps per CTA, [2] dynamic shared
  * memory in bytes, [3] staged kernel columns, [4] segments per group, [5] row pitch, [6] group stride
- * (floats), [7] groups per CTA, [8] lanes per row phase.  No counterpart in the reference. */
+ * (floats), [7] groups per CTA, [8] lanes per row phase, [9] lanes per CTA.  No counterpart in the reference. */
 int mlf_probe_conv_plan(int64_t W, int64_t H, int64_t n, int64_t kw, int32_t sms, int32_t smem_cta, int32_t smem_sm,
-                        int32_t variant, int64_t plan[9]);
+                        int32_t variant, int64_t plan[10]);
 
 /* Test support: the FP32 view kernel's launch shape of a solver.  plan[0], plan[1]: tile rows and
  * columns, plan[2]: channel slots per CTA, plan[3]: CTAs, plan[4]: partial planes that the reduction

@@ -572,7 +572,7 @@ int mlf_solver_destroy(mlf_solver* s) {
 int64_t mlf_solver_device_bytes(const mlf_solver* s) { return s ? (int64_t)s->bytes() : 0; }
 
 int mlf_probe_conv_plan(int64_t W, int64_t H, int64_t n, int64_t kw, int32_t sms, int32_t smem_cta, int32_t smem_sm,
-                        int32_t variant, int64_t plan[9]) {
+                        int32_t variant, int64_t plan[10]) {
   clear_error();
   if (!plan || W < 1 || H < 1 || n < 1 || kw < 1 || sms < 1)
     return fail(MLF_ERR_INVALID, "mlf_probe_conv_plan: empty call or null pointer");

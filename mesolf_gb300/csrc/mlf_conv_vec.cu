@@ -13,7 +13,8 @@
 // 15 kernels (one per x phase).  A thread owns SEG consecutive outputs x = 15 i + a of a segment of
 // 15 -- all its x phases a, or one half of them (a = 0..7 or 8..14, a CTA's threads the same half) --
 // in RPT rows y = b + 15 j of one slice; the (slice, row group, segment) triples of a phase are the
-// lanes of its CTAs, so warps are full whatever the sizes.  Per kernel row ky a CTA stages the input
+// lanes of its CTAs, so warps are full whatever the sizes (narrow images: further warps that only
+// stage).  Per kernel row ky a CTA stages the input
 // rows its lanes read and its kernels' row ky ([kx][a], padded to 16 or 8) in shared memory with
 // zero-filling cp.async, double buffered so that row ky + 1 loads while row ky is computed.  Along kx
 // the thread slides a window of inputs per row in registers (one new shared load per step and row)
@@ -64,7 +65,8 @@ struct ConvArgs {
   int kwp;                   // kernel columns walked: kw, or with whole segments the next multiple of 15 (zero taps)
   int SX, tilesX;            // segments per group and groups along x
   int width, pitch, gstride; // staged row: width = 15 SX + kwp - 1 floats, pitch apart; a group's RPT rows gstride
-  int max_groups;            // groups that a CTA's lanes can touch
+  int cta_lanes;             // lanes of a CTA, one per thread; further threads stage and compute nothing
+  int max_groups;            // groups that they can touch
   int64_t n;                 // slices
 };
 
@@ -85,9 +87,9 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
   const int nJ = b < A.H ? (A.H - b + CV_NN - 1) / CV_NN : 0;  // rows of this phase
   const int nP = (nJ + RPT - 1) / RPT;
   const int64_t lanes = A.n * nP * A.tilesX * A.SX;
-  const int64_t l0 = (int64_t)blockIdx.x * nthr;
+  const int64_t l0 = (int64_t)blockIdx.x * A.cta_lanes;
   if (l0 >= lanes) return;  // CTA-uniform
-  const int64_t lN = lanes < l0 + nthr ? lanes : l0 + nthr;
+  const int64_t lN = lanes < l0 + A.cta_lanes ? lanes : l0 + A.cta_lanes;
   const int64_t g0 = l0 / A.SX;
   const int ng = (int)((lN - 1) / A.SX - g0) + 1;  // <= max_groups
   auto group = [&](int64_t g, int& jp, int& xt) {  // -> slice
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(CV_MAX_THREADS) k_conv_vec_lanes(ConvArgs A) {
   }
   // this thread's lane
   const int64_t lane_id = l0 + tid;
-  const bool active = lane_id < lanes;
+  const bool active = tid < A.cta_lanes && lane_id < lanes;
   const int64_t g = active ? lane_id / A.SX : g0;
   const int il = active ? (int)(lane_id - g * A.SX) : 0;
   int jp, xt;
@@ -377,13 +379,14 @@ int64_t conv_lanes(const ConvArgs& a, int rpt) {
   return a.n * ((nJ + rpt - 1) / rpt) * (int64_t)a.tilesX * a.SX;
 }
 
-// Shared memory and group geometry of CTAs of `warps` warps; 0: they do not fit.
-size_t conv_fit(const ConvVariant& v, int warps, size_t budget, ConvArgs& c) {
+// Shared memory and group geometry of CTAs of `lanes` lanes; 0: they do not fit.
+size_t conv_fit(const ConvVariant& v, int lanes, size_t budget, ConvArgs& c) {
+  c.cta_lanes = lanes;
   c.kwp = v.halves == 2 ? c.kw : (c.kw + CV_NN - 1) / CV_NN * CV_NN;
   c.width = c.pitch = CV_NN * c.SX + c.kwp - 1;
   c.gstride = v.rpt * c.pitch;  // the next group's segments on the banks that follow (15 SX apart)
   while (c.gstride % 32 != (CV_NN * c.SX) % 32) ++c.gstride;
-  c.max_groups = (int)std::min<int64_t>((32 * warps + c.SX - 2) / c.SX + 1, (conv_lanes(c, v.rpt) + c.SX - 1) / c.SX);
+  c.max_groups = (int)std::min<int64_t>((lanes + c.SX - 2) / c.SX + 1, (conv_lanes(c, v.rpt) + c.SX - 1) / c.SX);
   // the rings read ahead, a few floats past their rows and taps: the last row's are past its group
   // where the stride has no padding
   constexpr size_t over = 64;
@@ -393,7 +396,7 @@ size_t conv_fit(const ConvVariant& v, int warps, size_t budget, ConvArgs& c) {
 }
 
 struct ConvPlan {
-  int variant = -1, warps = 0;
+  int variant = -1, warps = 0, lanes = 0;
   size_t smem = 0;
 };
 // Rows per thread, whole or half segments, and warps per CTA: those with the fewest cycles per
@@ -415,7 +418,7 @@ ConvPlan conv_plan(const ConvArgs& a, int nsm, int optin, int smem_sm, int only)
     const int64_t wp = (conv_lanes(a, v.rpt) + 31) / 32;  // warps per phase (and half)
     for (int k = 1; k <= CV_MAX_THREADS / 32; ++k) {
       ConvArgs c = a;
-      const size_t bytes = conv_fit(v, k, budget, c);
+      const size_t bytes = conv_fit(v, 32 * k, budget, c);
       if (!bytes) continue;
       const int64_t per_sm = std::max<int64_t>(1, std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (v.regs * 32 * k)));
       const int64_t ctas = CV_NN * v.halves * ((wp + k - 1) / k);
@@ -429,8 +432,28 @@ ConvPlan conv_plan(const ConvArgs& a, int nsm, int optin, int smem_sm, int only)
       const double cyc = (double)waves * (std::max(v.lone, v.each * (double)w) + (stage + 2.0) * (double)on_sm + 0.35 * k);
       if (p.variant < 0 || cyc < best) {
         best = cyc;
-        p = ConvPlan{i, k, bytes};
+        p = ConvPlan{i, k, 32 * k, bytes};
       }
+    }
+  }
+  // A warp of lanes on a narrow image has 32 / SX rows of its own to stage, one after the other, per
+  // kernel row.  Where all CTAs still run at once, warps without lanes share them: 31 x 31 x 60, kw 15
+  // 85 -> 66 us, 45 x 45 x 60, kw 25 114 -> 81, 62 x 62 x 40, kw 15 79 -> 72 with 64 lanes, 31 x 31 x 30,
+  // kw 21 101 -> 68 with eight warps; not in two waves (39 x 344 x 17, kw 220: 1622 -> 1942) nor on wider
+  // images (253 x 198 x 4, kw 136, 17 segments: 509 -> 578; 100 x 100 x 60, kw 15, 7 segments: 104 -> 109).
+  if (p.variant >= 0 && conv_variants()[p.variant].halves == 2 && a.SX <= 6 && conv_lanes(a, 1) > 32) {
+    const ConvVariant& v = conv_variants()[p.variant];
+    const int64_t lanes = conv_lanes(a, 1);
+    const bool few = CV_NN * 2 * ((lanes + 31) / 32) <= 2 * (int64_t)nsm;  // at most two warps of lanes per SM
+    const int shapes[3][2] = {{32, 8}, {32, 4}, {64, 4}};  // lanes, warps
+    for (int i = few ? 0 : 1; i < 3; ++i) {
+      ConvArgs c = a;
+      const size_t bytes = conv_fit(v, shapes[i][0], budget, c);
+      if (!bytes) continue;
+      const int64_t per_sm = std::min<int64_t>(smem_sm / (int64_t)(bytes + 10 * 1024), 65536 / (v.regs * 32 * shapes[i][1]));
+      if (CV_NN * 2 * ((lanes + shapes[i][0] - 1) / shapes[i][0]) > nsm * per_sm) continue;
+      p = ConvPlan{p.variant, shapes[i][1], shapes[i][0], bytes};
+      break;
     }
   }
   return p;
@@ -439,15 +462,15 @@ ConvPlan conv_plan(const ConvArgs& a, int nsm, int optin, int smem_sm, int only)
 }  // namespace
 
 int conv_plan_probe(int64_t W, int64_t H, int64_t n, int64_t kw, int nsm, int optin, int smem_sm, int variant,
-                    int64_t out[9]) {
+                    int64_t out[10]) {
   ConvArgs a = conv_sizes(W, H, n, kw);
   const ConvPlan p = conv_plan(a, nsm, optin, smem_sm, variant);
   if (p.variant < 0) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
   const ConvVariant& v = conv_variants()[p.variant];
-  conv_fit(v, p.warps, (size_t)optin, a);
-  const int64_t o[9] = {p.variant, p.warps, (int64_t)p.smem, a.kwp, a.SX, a.pitch, a.gstride, a.max_groups,
-                        conv_lanes(a, v.rpt)};
-  std::copy(o, o + 9, out);
+  conv_fit(v, p.lanes, (size_t)optin, a);
+  const int64_t o[10] = {p.variant, p.warps, (int64_t)p.smem, a.kwp, a.SX, a.pitch, a.gstride, a.max_groups,
+                         conv_lanes(a, v.rpt), p.lanes};
+  std::copy(o, o + 10, out);
   return MLF_OK;
 }
 
@@ -468,9 +491,9 @@ int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const f
   const ConvPlan p = conv_plan(a, nsm, optin, smem_sm, -1);
   if (p.variant < 0) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: kernel row does not fit in shared memory");
   const ConvVariant& v = conv_variants()[p.variant];
-  conv_fit(v, p.warps, (size_t)optin, a);
+  conv_fit(v, p.lanes, (size_t)optin, a);
   const int threads = 32 * p.warps;
-  const int64_t ctas = (conv_lanes(a, v.rpt) + threads - 1) / threads;
+  const int64_t ctas = (conv_lanes(a, v.rpt) + p.lanes - 1) / p.lanes;
   if (ctas > INT32_MAX) return fail(MLF_ERR_UNSUPPORTED, "direct MEX projector: too many slices");
   MLF_TRY(allow_max_dyn_smem(v.kernel));
   void* args[] = {&a};

@@ -281,7 +281,7 @@ int filter_run(Solver* s, cudaStream_t st);
 int conv_vec_run(const float* d_bitmap, int64_t W, int64_t H, int64_t n, const float* d_kernels,
                  int64_t kw, int nnum, float* d_out, cudaStream_t st);
 int conv_plan_probe(int64_t W, int64_t H, int64_t n, int64_t kw, int nsm, int optin, int smem_sm, int variant,
-                    int64_t out[9]);
+                    int64_t out[10]);
 // pieces of the tensor-core route of the MEX projector (mlf_conv_vec.cu)
 int summary_run(const float* dY, int64_t P, int64_t T, int mode, int bg_iter, int w1, int w2, int poly,
                 float* d_img, float* d_s, float* d_t, double* pass_ms, cudaStream_t st);

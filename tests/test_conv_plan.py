@@ -13,7 +13,7 @@ TAPS = {0: 8, 1: 16}  # floats per kernel column of the staged taps
 
 
 def conv_plan(lib, W, H, n, kw, variant):
-    p = (ctypes.c_int64 * 9)()
+    p = (ctypes.c_int64 * 10)()
     rc = lib.mlf_probe_conv_plan(W, H, n, kw, SMS, SMEM_CTA, SMEM_SM, variant, p)
     return list(p) if rc == _lib.MLF_OK else None
 
@@ -36,8 +36,9 @@ def test_reads_stay_inside_shared_memory(lib, variant):
                 p = conv_plan(lib, W, H, n, kw, variant)
                 if p is None:
                     continue  # one variant alone need not fit
-                v, warps, smem, kwp, SX, pitch, gstride, groups, lanes = p
+                v, warps, smem, kwp, SX, pitch, gstride, groups, lanes, cta_lanes = p
                 assert v == variant and 1 <= warps <= 12 and smem <= SMEM_CTA
+                assert 1 <= cta_lanes <= 32 * warps and groups * SX + SX > min(cta_lanes, lanes)
                 assert 4 * (last_read(v, kwp, SX, pitch, gstride, groups) + 1) <= smem, (W, H, n, kw)
 
 
@@ -46,3 +47,12 @@ def test_every_call_has_a_plan(lib):
     for W, H, n in ((1, 1, 1), (7, 3000, 1), (15, 16, 4000), (16, 16, 1), (500, 3, 9), (4000, 4000, 1)):
         for kw in (1, 2, 30, 135, 136, 340, 341):
             assert conv_plan(lib, W, H, n, kw, -1), (W, H, n, kw)
+
+
+def test_narrow_images_get_staging_warps(lib):
+    # at most six segments a row and room on the SMs: one warp of lanes, the others stage only
+    assert conv_plan(lib, 31, 31, 60, 15, -1)[1::8] == [4, 32]
+    assert conv_plan(lib, 31, 31, 30, 21, -1)[1::8] == [8, 32]
+    for W, H, n, kw in ((253, 198, 4, 136), (100, 100, 60, 15), (40, 35, 2, 21)):
+        p = conv_plan(lib, W, H, n, kw, -1)
+        assert p[9] == 32 * p[1]
