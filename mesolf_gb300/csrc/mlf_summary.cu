@@ -152,7 +152,7 @@ k_si_tnorm(const float* __restrict__ t_part, int ps, int64_t T, const float* __r
       v = s;
       l += e;
     }
-    t[j] = v + l;
+    t[j] = isfinite(v) ? v + l : v;  // two_sum leaves NaN in l beside an infinite sum
   }
   __syncthreads();
   if (tid < NS) {
