@@ -247,6 +247,7 @@ k_si_rowdot1(const float* __restrict__ Y, int64_t P, int64_t T, const float* __r
 // frames of 4 MB, 4.9 with 500 frames of 0.8 MB).  The two-pass form reads the movie once for s and
 // once for t, at 6.4 and 5.7 TB/s; this reads it once: 1.97 ms against 1.26 + 1.41 at
 // 1005 x 1005 x 2000, 0.83 against 1.36 with 1000 frames, 85 us against 66 + 86 at 465 x 450 x 500.
+// With fewer than 128 frames a block's fixed latency, about 1 us, outweighs what it reads (power_fit).
 // With more than 8 x 256 frames (32-pixel pieces: 4.3 against 4.0 ms at 1005 x 1005 x 3000) the two
 // passes stay.  The tile of the block in work is in registers, so all three 68 KB stages are in
 // flight.  The threads that publish s copy nothing: the release of a cluster barrier waits for the
@@ -683,7 +684,13 @@ int summary_block(int64_t T, int w1, int w2, size_t smem_max, size_t* smem) {
 
 namespace {
 // One power iteration in one pass (k_si_power): CTAs per cluster, frames per CTA and clusters;
-// clusters = 0 where it does not apply (a movie off the 16-byte grid, more than 2048 frames).
+// clusters = 0 where it does not apply (a movie off the 16-byte grid, more than 2048 frames) or the two
+// passes are faster: below 128 frames, but for movies of a few blocks per cluster, whose two launches
+// cost more than the blocks, and from 96 frames for movies far beyond the L2, whose second read comes
+// from HBM.  One pass against two, all of summary_image: 1005 x 1005 px, 16 frames 955 / 608 us, 64
+// 1267 / 1161, 96 (388 MB) 1560 / 1587, 128 1731 / 1886; 700 x 700, 32 700 / 504, 96 (188 MB) 969 / 937,
+// 128 1064 / 1090; 465 x 450, 16 495 / 414, 96 623 / 579, 160 707 / 736; 165 x 165 (three blocks), 8 393 /
+// 405, 96 423 / 429.
 struct PowerPlan {
   int cluster = 1, rows = 0, clusters = 0;
 };
@@ -706,6 +713,7 @@ int power_fit(PowerPlan* pp, int64_t P, int64_t T) {
   int nc = 0;
   MLF_CUDA(cudaOccupancyMaxActiveClusters(&nc, k_si_power, &cfg));
   if (nc < 1) return MLF_OK;
+  if (T < 128 && !(T >= 96 && 4 * P * T >= 230000000) && cdiv(P, SP_PB) > 3 * (int64_t)nc) return MLF_OK;
   pp->cluster = c;
   pp->rows = (int)cdiv(T, c);
   pp->clusters = (int)std::min<int64_t>(nc, cdiv(P, SP_PB));
