@@ -581,6 +581,24 @@ k_si_pixelwise(const float* __restrict__ Y, int64_t P, int T, const float* __res
   if (threadIdx.x == 0) img_max_part[blockIdx.x] = r;
 }
 
+// 1 / |t| and the mean of the FP32 t, for k_si_global (one block; in each of its blocks the FP64 sums
+// took a third of its 133 us at 1005 x 1005 x 16).
+__global__ void __launch_bounds__(SI_ROW_THREADS) k_si_tstat(const float* __restrict__ t, int64_t T, double* __restrict__ tn) {
+  __shared__ double shd[32];
+  double n2 = 0.0, m = 0.0;
+  for (int64_t j = threadIdx.x; j < T; j += SI_ROW_THREADS) {
+    const double v = __ldg(t + j);
+    n2 += v * v;
+    m += v;
+  }
+  n2 = block_sum(n2, shd);
+  m = block_sum(m, shd);
+  if (threadIdx.x == 0) {
+    tn[0] = 1.0 / sqrt(n2);
+    tn[1] = m / (double)T;
+  }
+}
+
 // Last pass, 'global': s and compute_std_image(Y/M, s, t) as written in the reference.  The
 // expansion cancels terms of the size of mean(y)^2 against each other, so sum(y^2), sum(y)
 // and s carry TwoSum compensation (s also the exact product error) and the formula runs in
@@ -589,25 +607,9 @@ k_si_pixelwise(const float* __restrict__ Y, int64_t P, int T, const float* __res
 // 3e-6 into the image at 140 frames.
 __global__ void __launch_bounds__(SI_ROW_THREADS)
 k_si_global(const float* __restrict__ Y, int64_t P, int64_t T, const float* __restrict__ t,
-            const float* __restrict__ scal, float* __restrict__ s_out, float* __restrict__ img,
-            float* __restrict__ img_max_part) {
+            const float* __restrict__ scal, const double* __restrict__ tn, float* __restrict__ s_out,
+            float* __restrict__ img, float* __restrict__ img_max_part) {
   __shared__ float sh[32];
-  __shared__ double shd[32], tn[2];
-  {
-    double n2 = 0.0, m = 0.0;
-    for (int64_t j = threadIdx.x; j < T; j += SI_ROW_THREADS) {
-      const double v = __ldg(t + j);
-      n2 += v * v;
-      m += v;
-    }
-    n2 = block_sum(n2, shd);
-    m = block_sum(m, shd);
-    if (threadIdx.x == 0) {
-      tn[0] = 1.0 / sqrt(n2);
-      tn[1] = m / (double)T;
-    }
-    __syncthreads();
-  }
   const int64_t p = (int64_t)blockIdx.x * SI_ROW_THREADS + threadIdx.x;
   float v_img = -INFINITY;
   if (p < P) {
@@ -789,18 +791,19 @@ int summary_run(const float* dY, int64_t P, int64_t T, int mode, int bg_iter, in
   const int64_t nrow = cdiv(P, nt);
   // one allocation for the scratch (each costs a call and, at its release, a device
   // synchronisation), every part 16-byte aligned
-  const int64_t parts[6] = {T + 4, std::max<int64_t>(ps, pp.clusters) * T, ps * ngrp, SC_N,
-                            std::max(nrow, cdiv(P, SI_ROW_THREADS)), P};
-  int64_t off[7] = {0};
-  for (int k = 0; k < 6; ++k) off[k + 1] = off[k] + (parts[k] + 3) / 4 * 4;
+  const int64_t parts[7] = {T + 4, std::max<int64_t>(ps, pp.clusters) * T, ps * ngrp, SC_N,
+                            std::max(nrow, cdiv(P, SI_ROW_THREADS)), P, 4};
+  int64_t off[8] = {0};
+  for (int k = 0; k < 7; ++k) off[k + 1] = off[k] + (parts[k] + 3) / 4 * 4;
   DevBuf scratch;
-  MLF_TRY(scratch.alloc(sizeof(float) * off[6], "summary: scratch"));
+  MLF_TRY(scratch.alloc(sizeof(float) * off[7], "summary: scratch"));
   float* const tb = scratch.as<float>();
   float* const tpart = tb + off[1];
   float* const maxpart = tb + off[2];
   float* const sc = tb + off[3];
   float* const imgpart = tb + off[4];
   float* const s_tmp = tb + off[5];
+  double* const tn = reinterpret_cast<double*>(tb + off[6]);
   const dim3 cgrid((unsigned)ngrp, (unsigned)ps);
   MLF_TRY(clk.mark(st));
   for (int it = 0; it < bg_iter; ++it) {
@@ -843,7 +846,9 @@ int summary_run(const float* dY, int64_t P, int64_t T, int mode, int bg_iter, in
     nparts = nrow;
   } else {
     nparts = cdiv(P, SI_ROW_THREADS);
-    k_si_global<<<(unsigned)nparts, SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, d_s, d_img, imgpart);
+    k_si_tstat<<<1, SI_ROW_THREADS, 0, st>>>(tb, T, tn);
+    MLF_LAUNCHED();
+    k_si_global<<<(unsigned)nparts, SI_ROW_THREADS, 0, st>>>(dY, P, T, tb, sc, tn, d_s, d_img, imgpart);
   }
   MLF_LAUNCHED();
   MLF_TRY(clk.mark(st));
