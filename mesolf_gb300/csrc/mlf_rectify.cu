@@ -523,9 +523,12 @@ int rectify_run(const void* d_raw, int dtype, int64_t total, int64_t fstride, in
   const size_t smem = 2 * (size_t)RR_SF * maxc * slot * es;  // two stage buffers
   const int64_t gx = (out_h + rows - 1) / rows, gy = (out_w + RR_COLS - 1) / RR_COLS;
   const int64_t stages = (n_out + RR_SF - 1) / RR_SF;
-  // the gather takes averaged frames, raw buffers off the 16-byte grid and pitches whose tiles
-  // would leave fewer than two blocks on an SM
-  const bool staged = navg == 1 && reinterpret_cast<uintptr_t>(d_raw) % 16 == 0 && smem <= 112 * 1024 && gy <= 65535;
+  // the gather takes averaged frames, raw buffers off the 16-byte grid, pitches whose tiles
+  // would leave fewer than two blocks on an SM, and 32-bit frames from pitch 1.1 on, whose large tiles
+  // leave few warps on an SM (1000 x 1000 x 200, pitch 1.2: 774 us against 1127 staged; 1.1: 827 against
+  // 961; at 1.02 941 against 1090, but there the staged kernel's rounding is kept; 0.8: 1276 against 1030)
+  const bool staged = navg == 1 && reinterpret_cast<uintptr_t>(d_raw) % 16 == 0 && smem <= 112 * 1024 && gy <= 65535 &&
+                      !(dtype == MLF_DTYPE_F32 && dx >= 1.1 * M);
   // calls that the 128 x 4 tiles of 16 frames took were limited to 65535 such stages: still refused
   if (staged && n_out > (int64_t)16 * 65535) {
     int rows4 = 0, cols4 = 0;
