@@ -527,10 +527,13 @@ int rectify_run(const void* d_raw, int dtype, int64_t total, int64_t fstride, in
   // would leave fewer than two blocks on an SM, and 32-bit frames from pitch 1.1 on, whose large tiles
   // leave few warps on an SM (1000 x 1000 x 200, pitch 1.2: 774 us against 1127 staged; 1.1: 827 against
   // 961; at 1.02 941 against 1090, but there the staged kernel's rounding is kept; 0.8: 1276 against 1030)
-  const bool staged = navg == 1 && reinterpret_cast<uintptr_t>(d_raw) % 16 == 0 && smem <= 112 * 1024 && gy <= 65535 &&
+  const int64_t hx = (out_h + RC_ROWS - 1) / RC_ROWS, hy = (out_w + RC_COLS - 1) / RC_COLS;  // the gather's blocks
+  const bool aligned = reinterpret_cast<uintptr_t>(d_raw) % 16 == 0;
+  const bool staged = navg == 1 && aligned && smem <= 112 * 1024 && hy <= 65535 &&
                       !(dtype == MLF_DTYPE_F32 && dx >= 1.1 * M);
-  // calls that the 128 x 4 tiles of 16 frames took were limited to 65535 such stages: still refused
-  if (staged && n_out > (int64_t)16 * 65535) {
+  // calls that the 128 x 4 tiles of 16 frames took were limited to 65535 such stages: still refused,
+  // whichever kernel takes them now
+  if (navg == 1 && aligned && hy <= 65535 && n_out > (int64_t)16 * 65535) {
     int rows4 = 0, cols4 = 0;
     for (int64_t r0 = 0; r0 < out_h; r0 += 128)
       rows4 = std::max(rows4, iy[std::min<int64_t>(r0 + 128, out_h) - 1] + 2 - iy[r0]);
@@ -567,7 +570,6 @@ int rectify_run(const void* d_raw, int dtype, int64_t total, int64_t fstride, in
     }
   } else {
     const int64_t per_block = (int64_t)RC_FCH * RC_NCH;
-    const int64_t hx = (out_h + RC_ROWS - 1) / RC_ROWS, hy = (out_w + RC_COLS - 1) / RC_COLS;
     const int64_t hz = (n_out + per_block - 1) / per_block;
     if (hz > 65535 || hy > 65535)
       return fail(MLF_ERR_UNSUPPORTED, "mlf_rectify_frames: too many output frames or columns for one launch");
