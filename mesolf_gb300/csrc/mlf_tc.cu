@@ -1504,8 +1504,10 @@ k_tc_im2col(const float* __restrict__ R, const int* __restrict__ tile_patch, con
 // consecutive positions (lanes); warp w takes the tap rows db = w, w+16, ..., so each load of
 // a warp is 32 consecutive floats of one tap's row.  Bound: latency of L2 reads, so the columns of
 // a tap row go in groups of sixteen independent loads (out-of-range ones predicated off): 40 -> 19 us
-// with eight and 17 with sixteen for 59136 positions with one split, 18.7 -> 7.9 for 3200 with six.  Sums in a fixed order
-// (deterministic).  rmax (nullable, FP16 modes) receives max |R|.
+// with eight and 17 with sixteen for 59136 positions with one split, 18.7 -> 7.9 for 3200 with six.  Few taps
+// leave warps without a tap row and most of the sixteen loads unused, so below T 8 the splits go over the
+// warps too and a thread takes two or four of them at once: bf16x2, four iterations of 30 x 30 x 7, T 3, 14.5 ->
+// 11.8 ms, 20 x 30 x 11, T 5, 11.6 -> 9.0, two of 26 x 33 x 16, T 7, 6.25 -> 5.61.  Sums in a fixed order (deterministic).  rmax (nullable, FP16 modes) receives max |R|.
 constexpr int COL2IM_WARPS = 16;
 // The positions from pos0 on that ypart holds (MP of them), of the views blockIdx.y: their partials
 // vstride and their outputs hx_stride floats apart.
@@ -1539,20 +1541,48 @@ k_tc_col2im_ratio(const float* __restrict__ ypart, int splits, int MP, int NB, i
     const int q = (T - 1) / 2;
     const int64_t sstride = (int64_t)NB * MP;
     const int da_lo = max(0, q - i), da_hi = min(T - 1, Li - 1 - i + q);  // 0 <= i + da - q < Li
-    for (int db = w; db < T; db += COL2IM_WARPS) {
-      const int b = j + db - q;
-      if (b < 0 || b >= Lj) continue;
-      // element (db, da): (db*T + da)*MP + pos0 + b*Li + i + da - q
-      const float* yrow = ypart + (int64_t)(db * T) * MP + (pos0 - pr.pos0) + (int64_t)b * Li + (i - q);
-      for (int sp = 0; sp < splits; ++sp, yrow += sstride) {
-        for (int d0 = 0; d0 < T; d0 += 16) {
+    // element (db, da): (db*T + da)*MP + pos0 + b*Li + i + da - q
+    auto row = [&](int db, int b) {
+      return ypart + (int64_t)(db * T) * MP + (pos0 - pr.pos0) + (int64_t)b * Li + (i - q);
+    };
+    if (T < 8) {
+      // group w / T of the warps, splits w / T, + groups, ...: NS splits of CW columns at a time
+      const int groups = COL2IM_WARPS / T, db = w % T, g = w / T, b = j + db - q;
+      const float* yrow = row(db, b);
+      auto sum = [&](auto cw) {
+        constexpr int CW = decltype(cw)::value, NS = 16 / CW;
+        for (int sp = g; sp < splits; sp += NS * groups) {
           float v[16];
 #pragma unroll
-          for (int u = 0; u < 16; ++u)
-            v[u] = (d0 + u >= da_lo && d0 + u <= da_hi) ? __ldg(yrow + (int64_t)(d0 + u) * (MP + 1)) : 0.f;
+          for (int u = 0; u < 16; ++u) {
+            const int k = sp + u / CW * groups, da = u % CW;
+            v[u] = (k < splits && da >= da_lo && da <= da_hi) ? __ldg(yrow + k * sstride + (int64_t)da * (MP + 1)) : 0.f;
+          }
 #pragma unroll
-          for (int u = 0; u < 16; u += 8)
-            s += ((v[u] + v[u + 1]) + (v[u + 2] + v[u + 3])) + ((v[u + 4] + v[u + 5]) + (v[u + 6] + v[u + 7]));
+          for (int u = 0; u < 16; u += 4) s += (v[u] + v[u + 1]) + (v[u + 2] + v[u + 3]);
+        }
+      };
+      if (g < groups && b >= 0 && b < Lj) {
+        if (T <= 4)
+          sum(std::integral_constant<int, 4>());
+        else
+          sum(std::integral_constant<int, 8>());
+      }
+    } else {
+      for (int db = w; db < T; db += COL2IM_WARPS) {
+        const int b = j + db - q;
+        if (b < 0 || b >= Lj) continue;
+        const float* yrow = row(db, b);
+        for (int sp = 0; sp < splits; ++sp, yrow += sstride) {
+          for (int d0 = 0; d0 < T; d0 += 16) {
+            float v[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u)
+              v[u] = (d0 + u >= da_lo && d0 + u <= da_hi) ? __ldg(yrow + (int64_t)(d0 + u) * (MP + 1)) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 16; u += 8)
+              s += ((v[u] + v[u + 1]) + (v[u + 2] + v[u + 3])) + ((v[u + 4] + v[u + 5]) + (v[u + 6] + v[u + 7]));
+          }
         }
       }
     }
