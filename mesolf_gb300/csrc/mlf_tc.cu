@@ -41,6 +41,7 @@
 #include <map>
 #include <memory>
 #include <queue>
+#include <set>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -1820,9 +1821,12 @@ size_t tc_psf_bytes(const Psf* p) {
 
 size_t tc_work_bytes(const TcSolverState* t) {
   if (!t) return 0;
+  size_t items = 0;
+  for (const auto& i : t->items) items += i.second.tab.bytes;
   return t->X.bytes + t->lfs.bytes + t->rimg.bytes + t->tile_patch.bytes + t->pinfo.bytes + t->wtab_dev.bytes +
          t->wscratch.bytes + t->ar_hi.bytes + t->ar_lo.bytes + t->a1.bytes +
-         t->ypart.bytes + t->err.bytes + t->Xprev.bytes + t->relbuf.bytes + t->a1h.bytes + t->f16s.bytes;
+         t->ypart.bytes + t->err.bytes + t->Xprev.bytes + t->relbuf.bytes + t->a1h.bytes + t->f16s.bytes +
+         items;
 }
 
 size_t tc_solver_bytes(const Solver* s) { return tc_work_bytes(s->tc); }
@@ -1860,6 +1864,26 @@ std::vector<ItemCost> item_costs(int NN, int KB, int NB, const std::vector<int>&
         out.push_back({drain + tile * (r.n_hi - r.n_lo), m * splits + s});
       }
   return out;
+}
+// The item table of the fused view step for a split count: entry c + k * grid is the k-th item of CTA c, -1
+// for none.
+struct ItemTable {
+  int grid = 0;
+  std::vector<int> tab;
+};
+ItemTable item_table(int NN, int KB, int NB, const std::vector<int>& tiles, const std::vector<int>& z0,
+                     const std::vector<int>& nz, int splits, int nsm) {
+  const std::vector<ItemCost> costs = item_costs(NN, KB, NB, tiles, z0, nz, splits);
+  ItemTable t;
+  t.grid = std::min((int)costs.size(), nsm);
+  std::vector<std::vector<int>> lists(t.grid);
+  assign_items(costs, t.grid, &lists);
+  size_t rounds = 0;
+  for (const auto& l : lists) rounds = std::max(rounds, l.size());
+  t.tab.assign(rounds * t.grid, -1);
+  for (int c = 0; c < t.grid; ++c)
+    for (size_t k = 0; k < lists[c].size(); ++k) t.tab[k * t.grid + c] = lists[c][k];
+  return t;
 }
 // Splits of the forward GEMM.  The fused view step's items are (position tile, split), so the split
 // count sets how evenly they fill the CTAs: the count with the shortest makespan plus the time
@@ -1908,13 +1932,20 @@ size_t tc_work_plan_bytes(const Psf* psf, const std::vector<int>& Li, const std:
     MP += rup(Li[p] * Lj[p], BM);
     tiles += rup(Li[p] * Lj[p], BM) / BM;
   }
-  const SplitPlan sp = plan_splits(psf->N * psf->N, rup((psf->T + 2) * (psf->T + 2), BK), NB, Li, Lj, z0, nz, nsm);
+  const SplitPlan sp = plan_splits(psf->N * psf->N, KB, NB, Li, Lj, z0, nz, nsm);
+  // the item tables of the split counts that the autotuner tries
+  std::vector<int> ptiles;
+  for (size_t p = 0; p < Li.size(); ++p) ptiles.push_back((Li[p] * Lj[p] + BM - 1) / BM);
+  size_t items = 0;
+  for (int s : std::set<int>{std::max(1, sp.def / 2), sp.def, sp.max})
+    items += sizeof(int) * item_table(psf->N * psf->N, KB, NB, ptiles, z0, nz, s, nsm).tab.size();
   const int64_t P = (int64_t)Li.size();
   return (size_t)(psf->nch * MP * 4 + (int64_t)psf->N * psf->N * MP * 4 + MP * 4 + tiles * 4 + 8 * P * 4 +
                   (int64_t)psf->N * psf->N * P * 4 + P * 4 + 4 * MP * KB * 2 + 16 +
                   (int64_t)sp.max * MP * NB * 4 + 4 +
                   // convergence monitor, allocated by the first solve that asks for stats
-                  psf->nch * MP * 4 + (int64_t)kRelChangeBufDoubles * 8);
+                  psf->nch * MP * 4 + (int64_t)kRelChangeBufDoubles * 8) +
+         items;
 }
 
 int tc_work_create(Psf* psf, const std::vector<Solver*>& members, TcSolverState** out, cudaStream_t st) {
@@ -2227,19 +2258,12 @@ int tc_items(const Psf* psf, TcSolverState* t) {
   if (t->items.count(t->splits)) return MLF_OK;
   std::vector<int> tiles;
   for (int p = 0; p < t->P; ++p) tiles.push_back((t->LL[p] + BM - 1) / BM);
-  const std::vector<ItemCost> costs =
-      item_costs(psf->N * psf->N, psf->tc->KB, psf->tc->NB, tiles, t->z0, t->nz, t->splits);
-  const int grid = std::min((int)costs.size(), t->nsm);
-  std::vector<std::vector<int>> lists(grid);
-  assign_items(costs, grid, &lists);
-  size_t rounds = 0;
-  for (const auto& l : lists) rounds = std::max(rounds, l.size());
-  std::vector<int> tab(rounds * grid, -1);
-  for (int c = 0; c < grid; ++c)
-    for (size_t k = 0; k < lists[c].size(); ++k) tab[k * grid + c] = lists[c][k];
+  const ItemTable it =
+      item_table(psf->N * psf->N, psf->tc->KB, psf->tc->NB, tiles, t->z0, t->nz, t->splits, t->nsm);
+  const std::vector<int>& tab = it.tab;
   TcSolverState::Items& e = t->items[t->splits];
   e.n = (int)tab.size();
-  e.grid = grid;
+  e.grid = it.grid;
   e.identity = true;
   for (size_t k = 0; k < tab.size(); ++k) e.identity = e.identity && tab[k] == (int)k;
   int rc = e.tab.alloc(tab.size() * sizeof(int), "tc item table");
