@@ -2254,7 +2254,7 @@ bool tc_fused_ok(const Psf* psf, const TcSolverState* t, int precision) {
 
 // The fused view step's item table for the split count in use, built on first use (it allocates:
 // outside any capture) and kept with the work set.
-int tc_items(const Psf* psf, TcSolverState* t) {
+int tc_items(const Psf* psf, TcSolverState* t, cudaStream_t st) {
   if (t->items.count(t->splits)) return MLF_OK;
   std::vector<int> tiles;
   for (int p = 0; p < t->P; ++p) tiles.push_back((t->LL[p] + BM - 1) / BM);
@@ -2267,7 +2267,10 @@ int tc_items(const Psf* psf, TcSolverState* t) {
   e.identity = true;
   for (size_t k = 0; k < tab.size(); ++k) e.identity = e.identity && tab[k] == (int)k;
   int rc = e.tab.alloc(tab.size() * sizeof(int), "tc item table");
-  if (rc == MLF_OK && cudaMemcpy(e.tab.p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+  // on the solve's stream: a plain copy from pageable memory may still be under way when it returns, and
+  // nothing orders a stream that does not synchronise with the default one behind it
+  if (rc == MLF_OK && (cudaMemcpyAsync(e.tab.p, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+                       cudaStreamSynchronize(st) != cudaSuccess))
     rc = fail(MLF_ERR_CUDA, "tc item table upload");
   if (rc != MLF_OK) t->items.erase(t->splits);
   return rc;
@@ -2468,7 +2471,7 @@ int tc_autotune(const Psf* psf, TcSolverState* t, int precision, cudaStream_t st
     t->splits = sp;
     float ms = 0.f;
     if (fused) {
-      MLF_TRY(tc_items(psf, t));
+      MLF_TRY(tc_items(psf, t, st));
       MLF_TRY(timed([&]() -> int {
         MLF_TRY(tc_bwdfwd_launch(psf, t, precision, v0, t->views[1], w0, w0 + t->P, st));
         return tc_col2im(psf, t, t->views[1], false, nullptr, st, precision, 0);
@@ -2588,7 +2591,7 @@ int tc_run(TcSolverState* t, const std::vector<Solver*>& members, const std::vec
   if (max_iter > 0) {
     MLF_TRY(tc_autotune(psf, t, precision, st));  // first solve at this precision only
     tc_apply_tune(t, precision);
-    if (tc_fused_ok(psf, t, precision)) MLF_TRY(tc_items(psf, t));
+    if (tc_fused_ok(psf, t, precision)) MLF_TRY(tc_items(psf, t, st));
     if (monitor) MLF_CUDA(cudaMemcpyAsync(t->Xprev.p, t->X.p, t->X.bytes, cudaMemcpyDeviceToDevice, st));
     TcSolverState::Iteration& g = t->iter[precision][timer->timing ? 1 : 0];
     if (!g.exec) {
