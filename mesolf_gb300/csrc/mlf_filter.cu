@@ -40,8 +40,9 @@ struct FGeo {
 
 // FP64 runs at two operations per SM and cycle here, conversions no faster, so the two uses that
 // touch every voxel are kept off it: sums are pairs of floats (each addition's rounding error, exact by
-// TwoSum, goes to the second one; about 48 bits, then FP64 across threads), and the scaling multiplies
-// by a pair, rounding the product once.  45 x 70 x 51 lenslets: row pass 437 -> 350 us, column pass
+// TwoSum, goes to the second one; about 48 bits, then FP64 across threads; where a thread's sum leaves the
+// floats' range, the block sums again in FP64), and the scaling multiplies by a pair, rounding the product
+// once.  45 x 70 x 51 lenslets: row pass 437 -> 350 us, column pass
 // 435 -> 367, k_rephase 205 -> 74.
 struct PairSum {
   float s = 0.f, e = 0.f;
@@ -50,8 +51,9 @@ struct PairSum {
     e += (s - (t - b)) + (v - b);
     s = t;
   }
-  // an overflow or a value that is not finite leaves NaN in e; the sum is then s
-  __device__ __forceinline__ double value() const { return isfinite(s) ? (double)s + (double)e : (double)s; }
+  // not finite: a value that was not, or a sum beyond the floats' range, which FP64 holds
+  __device__ __forceinline__ bool over() const { return !isfinite(s); }
+  __device__ __forceinline__ double value() const { return (double)s + (double)e; }
 };
 
 // MATLAB layout -> phase-major for the filtered planes, scaling each plane by scale[z]: one
@@ -75,7 +77,11 @@ __global__ void k_rephase(const float* __restrict__ V, FGeo f, const double* __r
   __syncthreads();
   // v * scale with scale = hi + lo: fma gives the rounding error of v * hi
   const double sc = scale[z];
-  const float hi = (float)sc, lo = isfinite(hi) ? (float)(sc - (double)hi) : 0.f;
+  if (!(fabs(sc) >= 0x1p-100 && fabs(sc) <= 0x1p100)) {  // no pair of floats holds it (0 and NaN too)
+    phase_lines_out(X, g, nl, g.Li, tab, lines, [sc](float v) { return (float)((double)v * sc); });
+    return;
+  }
+  const float hi = (float)sc, lo = (float)(sc - (double)hi);
   phase_lines_out(X, g, nl, g.Li, tab, lines, [hi, lo](float v) {
     const float p = v * hi, r = p + fmaf(v, lo, fmaf(v, hi, -p));
     return isfinite(r) ? r : p;
@@ -90,9 +96,9 @@ __global__ void k_rephase(const float* __restrict__ V, FGeo f, const double* __r
 // taps in groups of 8 over a 16-value register window, so one group costs 8 window loads
 // and 2 tap loads for 64 FMAs.  Every output adds its products in the order k = 0, 1, ...
 // (the zero taps add exactly nothing).
-// `emit(line, i0, values)` stores the outputs i0 .. i0 + 7 below L; returns the thread's FP64 sum of outputs.
+// `emit(line, i0, values)` stores the outputs i0 .. i0 + 7 below L; returns the thread's sum of outputs.
 template <class Emit>
-__device__ double filter_lines(const float* __restrict__ buf, int L, const float* __restrict__ taps,
+__device__ PairSum filter_lines(const float* __restrict__ buf, int L, const float* __restrict__ taps,
                                int ntp, int wlo, int nlines, Emit emit) {
   static_assert(kChunk == 8, "the register window assumes 8 outputs per thread");
   const int lane = threadIdx.x % kLines, half = threadIdx.x % 32 / kLines, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -140,7 +146,7 @@ __device__ double filter_lines(const float* __restrict__ buf, int L, const float
     for (int t = 0; t < kChunk; ++t)
       if (i0 + t < L) s.add(acc[t]);
   }
-  return s.value();
+  return s;
 }
 
 // Stage the taps of bank entry e in shared memory, zero-padded to a multiple of 8.
@@ -153,11 +159,20 @@ __device__ __forceinline__ int stage_taps(float* tsm, const float* __restrict__ 
 // shared-memory offset (floats) of the staged taps, after a line buffer of L lines
 __host__ __device__ constexpr int taps_offset(int L) { return (L * kPad + 3) & ~3; }
 
-__device__ void block_reduce_store(double s, double* out) {
+// The block's FP64 sum of p, or of again() where a thread's p left the floats' range; again() is called after a
+// barrier.
+template <class Again>
+__device__ __forceinline__ void block_reduce_store(const PairSum& p, double* out, Again again) {
   __shared__ double sh[32];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-  __syncthreads();
+  auto warps = [&](double s) {
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  };
+  warps(p.value());
+  if (__syncthreads_or(p.over())) {
+    warps(again());
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
     double r = 0.0;
     for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r += sh[i];
@@ -184,14 +199,17 @@ __global__ void k_filter_r(const float* __restrict__ X, PatchGeo pg, float* __re
   PairSum sin;
   phase_gather(X, pg, c0, z, nlines, 0, pg.Li, buf, kPad, 1, [&](float v) { sin.add(v); });
   __syncthreads();
-  double sout = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
+  filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
     // the pitch holds whole groups of four; its floats past the line are never read
     float* d = plane + (int64_t)(c0 + l) * g.Vp + i0;
     *reinterpret_cast<float4*>(d) = make_float4(y[0], y[1], y[2], y[3]);
     if (i0 + 4 < g.Vp) *reinterpret_cast<float4*>(d + 4) = make_float4(y[4], y[5], y[6], y[7]);
   });
-  (void)sout;
-  block_reduce_store(sin.value(), sums_in + (int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+  block_reduce_store(sin, sums_in + (int64_t)blockIdx.y * gridDim.x + blockIdx.x, [&]() {
+    double s = 0.0;
+    for (int i = threadIdx.x; i < L * nlines; i += blockDim.x) s += (double)buf[i / nlines * kPad + i % nlines];
+    return s;
+  });
 }
 
 // Pass along c (stride Xr): grid (ceil(Xr / kLines), Zf).  Lines = rows r of plane z.
@@ -225,12 +243,16 @@ __global__ void k_filter_c(float* __restrict__ V, FGeo g, const int* __restrict_
   }
   __syncthreads();
   const int L = (int)g.Xc;
-  double s = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
+  const PairSum sum = filter_lines(buf, L, tsm, ntp, wlo_e[e], nlines, [&](int l, int i0, const float (&y)[kChunk]) {
 #pragma unroll
     for (int t = 0; t < kChunk; ++t)
       if (i0 + t < L) plane[(int64_t)(i0 + t) * g.Vp + r0 + l] = y[t];
   });
-  block_reduce_store(s, sums_out + (int64_t)blockIdx.y * gridDim.x + blockIdx.x);
+  block_reduce_store(sum, sums_out + (int64_t)blockIdx.y * gridDim.x + blockIdx.x, [&]() {  // from the outputs
+    double s = 0.0;
+    for (int i = threadIdx.x; i < L * nlines; i += blockDim.x) s += (double)plane[(int64_t)(i / nlines) * g.Vp + r0 + i % nlines];
+    return s;
+  });
 }
 
 // scale[z] = sum_before / sum_after for filtered planes (fixed-order sums, one warp per plane), 1
