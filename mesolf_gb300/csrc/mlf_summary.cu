@@ -698,8 +698,14 @@ struct PowerPlan {
 };
 size_t power_smem(int64_t rows) { return sizeof(float) * SP_STAGES * (size_t)rows * (SP_PB + 4); }
 int power_fit(PowerPlan* pp, int64_t P, int64_t T) {
+  // clusters of 1, 2, 4, 5 and 8: eight CTAs for 1025 to 1280 frames are little more than half full, and their
+  // blocks take as long (1005 x 1005 x 1100: 8.85 ms, two passes 8.11, five CTAs 6.27).  Three and six
+  // are faster than four and eight too (x 520 3.47 and 3.99 ms), but leave t further off FP64 (330 x 300 x
+  // 560 4.4e-8 and 4.0e-8, 300 x 165 x 1400 4.7e-8 and 4.1e-8; five 4.5e-8 and 4.3e-8 at 165 x 165 x 1100,
+  // 4.7e-8 and 4.9e-8 at 450 x 420 x 1200, the two passes before 5e-8 to 7e-8)
   int c = 1;
-  while (c < SP_MAX_CLUSTER && cdiv(T, c) > SP_ROWS) c *= 2;
+  for (int size : {1, 2, 4, 5, SP_MAX_CLUSTER})
+    if (cdiv(T, c) > SP_ROWS) c = size;
   if (cdiv(T, c) > SP_ROWS || cdiv(T, c) * P >= ((int64_t)1 << 32)) return MLF_OK;
   MLF_TRY(allow_max_dyn_smem((const void*)k_si_power));
   cudaLaunchConfig_t cfg{};
