@@ -252,18 +252,22 @@ __global__ void k_scatter_views(const float* __restrict__ lfs, PatchGeo g, float
 // kReduceGroups, ... and their sums are added in a fixed order (deterministic).  Bound by the
 // latency of the L2 reads, so 32 warps share the planes (31 x 40 lenslets: 22.6 us for 1824
 // slot planes on 8 warps, 4.2 us for the 456 planes that the CTAs leave on 32).
-// The next view kernel may be launched once the sums are formed, so that its CTAs settle on SMs that the
-// view kernel before has left.  With the launch at this kernel's start they were placed while that one
-// still ran, and patches of middle size took up to half again as long (one iteration of 60 x 60 x 25
-// lenslets, T 11: 42.6 -> 28.4 ms, of 58 x 58 x 51, T 15: 143 -> 126, without dependent launches 28.8
-// and 126; four of 11 x 11 x 21, T 3: 5.35 -> 5.04, without 6.99).
+// The next view kernel is launched when the view kernel before has ended, so that its CTAs settle on SMs
+// that one has left: with the launch at this kernel's start they were placed while it still ran, and patches
+// of middle size took up to half again as long (one iteration of 60 x 60 x 25 lenslets, T 11: 42.6 -> 28.4
+// ms, of 58 x 58 x 51, T 15: 143 -> 126; without dependent launches 28.8 and 126).  `early`: right after
+// pdl_wait, for small patches (the small tile, or four and more slots per CTA), whose launches are what a
+// view step waits for; otherwise once the sums are formed.  Early against late: 11 x 11 x 21, T 3, four
+// iterations 4.89 / 5.08 ms (without 6.99), forward 16 x 25 x 22, T 9 5.51 / 5.85, 31 x 13 x 14 2.63 / 2.73;
+// 40 x 40 x 21, T 9 (three slots) 9.84 / 9.57, 60 x 60 x 25 29.5 / 28.4, 45 x 52 x 51, T 15 96.9 / 94.1.
 constexpr int kReduceGroups = 32;
 __global__ void __launch_bounds__(32 * kReduceGroups)
 k_reduce_ratio(const float* part, int nparts, int Li, int Lj, int HP, int64_t PPL,
                const float* __restrict__ lfsub, float* __restrict__ hx_out,
-               float* __restrict__ rpad, int RP, int off) {
+               float* __restrict__ rpad, int RP, int off, int early) {
   __shared__ float sh[kReduceGroups][32];
   pdl_wait();
+  if (early) pdl_launch_dependents();
   const int LL = Li * Lj;
   const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
@@ -449,9 +453,10 @@ int run_reduce(Solver* s, int view, float* hx_out, bool ratio, cudaStream_t st) 
   const int group = view_sums_slots(s->slots) ? s->slots : 1;  // planes that the view kernel has added
   const float* part = s->part.as<float>();
   int nparts = (int)view_partials(s), Li = s->Li, Lj = s->Lj, hp = HP, RP = s->RP, off = s->q + 1;
+  int early = s->small || s->slots >= 4;  // small patches: the comment at the kernel
   int64_t ppl = (int64_t)group * s->tilesB * s->tileY * HP;
   float* rpad = ratio ? s->rpad.as<float>() : nullptr;
-  void* args[] = {&part, &nparts, &Li, &Lj, &hp, &ppl, &lfsub, &hx_out, &rpad, &RP, &off};
+  void* args[] = {&part, &nparts, &Li, &Lj, &hp, &ppl, &lfsub, &hx_out, &rpad, &RP, &off, &early};
   MLF_CUDA(launch_pdl((const void*)k_reduce_ratio, ceil_div(LL, 32), 32 * kReduceGroups, args, 0, st));
   return MLF_OK;
 }
