@@ -1516,7 +1516,7 @@ struct PartRange {
   int pos0;
   int64_t vstride, hx_stride;
 };
-// FEW: T < 8.  A kernel of its own: in one with the general form it takes 40 registers for 32, a block less on
+// FEW: T < 8 (tc_col2im).  A kernel of its own: in one with the general form it takes 40 registers for 32, a block less on
 // an SM (forward projection 31 x 40 x 26, T 9, 5.57 -> 6.03 ms, 376 x 376 x 77 slices, kw 241, 18.9 -> 19.4).
 template <bool FEW>
 __global__ void __launch_bounds__(32 * COL2IM_WARPS)
@@ -2140,7 +2140,12 @@ int tc_col2im(const Psf* psf, TcSolverState* t, int view, bool ratio, float* hx_
   const int MP = (part.ntiles ? part.ntiles : t->MP / BM) * BM;
   const PartRange pr{part.tile0 * BM, (int64_t)t->splits * psf->tc->NB * MP, t->MP};
   float* rmax = (ratio && prec_f16(precision)) ? t->f16s.as<float>() + 1 + slot : nullptr;
-  auto kernel = psf->T < 8 ? k_tc_col2im_ratio<true> : k_tc_col2im_ratio<false>;
+  // few taps: where there are splits to go over the warps, and all blocks run at once whatever the registers
+  // (24 patches of 31-60 lenslets, T 7, one split 69.1 ms, general form 68.0; 12 patches, T 3, 800 blocks 28.2
+  // and 27.3; 400 x 400 x 60 slices, kw 75 11.4 and 10.8; 60 x 60 x 7, T 3, 116 blocks of five splits 10.2
+  // and 10.6)
+  const bool few = psf->T < 8 && t->splits > 2 && (MP + 31) / 32 <= 3 * t->nsm;
+  auto kernel = few ? k_tc_col2im_ratio<true> : k_tc_col2im_ratio<false>;
   kernel<<<dim3((MP + 31) / 32, part.nviews), 32 * COL2IM_WARPS, 0, st>>>(
       t->ypart.as<float>(), t->splits, MP, psf->tc->NB, psf->T, t->tile_patch.as<int>(), t->pinfo.as<int>(),
       t->lfs.as<float>() + (int64_t)view * t->MP, hx_out, ratio ? t->rimg.as<float>() : nullptr, rmax, pr);
