@@ -1069,7 +1069,8 @@ def summary_block(dev, side=1005, T=2000, steps=3, cpu=True, cpu_pixels=8192, e2
     T-frame sensor movie with the reference's default parameters (pixelwise detrend,
     bg_iter 5, windows 100 and 20 frames, poly_index 3), movie resident in HBM (`value`) and
     from pinned host memory (`e2e`).  The movie is 4 B x pixels x frames (8.08 GB at 1005^2 x
-    2000, larger than L2); every pass streams it once: 2 x bg_iter passes per call."""
+    2000, larger than L2); every pass streams it once: bg_iter + 1 passes per call where a power
+    iteration is one read (128 to 2048 frames), else 2 x bg_iter."""
     import torch
     from mesolf_gb300 import synth
     from mesolf_gb300.api import summary_image
@@ -1092,7 +1093,8 @@ def summary_block(dev, side=1005, T=2000, steps=3, cpu=True, cpu_pixels=8192, e2
     ms = e0.elapsed_time(e1) / steps
     acc /= steps
     movie_bytes = 4.0 * P * T
-    passes = 2 * prm[1]
+    one_read = 128 <= T <= 2048
+    passes = prm[1] + 1 if one_read else 2 * prm[1]
     hbm = _measured_hbm()
     gbs = lambda t_ms: movie_bytes / (t_ms * 1e-3) / 1e9 if t_ms > 0 else None
     last_gbs = gbs(acc[3])
@@ -1114,7 +1116,7 @@ def summary_block(dev, side=1005, T=2000, steps=3, cpu=True, cpu_pixels=8192, e2
            "movie_gb": movie_bytes / 1e9, "movie_passes": passes,
            "pass_ms": {"first_column_with_max": acc[0], "column": acc[1], "row": acc[2],
                        "last_pixelwise": acc[3], "finalise": acc[4]},
-           "stream_gbs": {"column": gbs(acc[1]), "row": gbs(acc[2]), "last_pixelwise": last_gbs,
+           "stream_gbs": {"column": None if one_read else gbs(acc[1]), "row": gbs(acc[2]), "last_pixelwise": last_gbs,
                           "whole_call": movie_bytes * passes / (ms * 1e-3) / 1e9},
            "roofline": {"bound": "hbm", "kernel": "k_si_pixelwise (last pass: s, moving means, power, std)",
                         "achieved": last_gbs, "peak": hbm, "unit": "GB/s",
@@ -1125,7 +1127,7 @@ def summary_block(dev, side=1005, T=2000, steps=3, cpu=True, cpu_pixels=8192, e2
            "e2e": {"value": T / t_e2e, "unit": "frames/s", "s_per_call": t_e2e,
                    "h2d_bytes_per_step": int(movie_bytes), "d2h_bytes_per_step": int(4 * (2 * P + T)),
                    "same_result_as_device_input": same},
-           "kernel_launches_per_call": 3 * prm[1] + 2,
+           "kernel_launches_per_call": (2 if one_read else 3) * prm[1] + (3 if one_read else 2),
            "data": "synthetic: per-pixel baselines, 20% bleaching trend, calcium-like transients, noise "
                    "(mesolf_gb300/synth.py sensor_movie)"}
     if cpu:

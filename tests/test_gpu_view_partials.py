@@ -20,8 +20,9 @@ pytestmark = pytest.mark.gpu
     ((67, 67), 61, 1, (4, 8), 2, 113),     # 225 channels, two slots of 160 threads
     ((24, 24), 61, 7, (2, 4), 2, 788),     # 1575 channels, the small tile
     ((71, 71), 61, 3, (4, 8), 1, None),    # one slot
-    ((11, 11), 61, 21, (2, 4), None, None),
-    ((30, 31), 91, 40, (4, 8), None, None),  # more than two slots: a CTA adds its own
+    ((11, 11), 61, 21, (2, 4), 10, 473),   # the last CTA has five of ten slots
+    ((41, 33), 91, 24, (4, 8), 3, None),   # three slots: a CTA adds its own
+    ((30, 31), 91, 40, (4, 8), 6, None),
 ])
 def test_no_plane_is_read_unwritten(cuda, lenslets, K0, Z, tile, slots, ctas):
     import torch
@@ -42,10 +43,7 @@ def test_no_plane_is_read_unwritten(cuda, lenslets, K0, Z, tile, slots, ctas):
     poison()
     assert (plan[0], plan[1]) == tile
     nch = 225 * Z
-    if slots is not None:
-        assert plan[2] == slots
-    else:
-        assert plan[2] > 2 or tile == (2, 4)
+    assert plan[2] == slots
     if ctas is not None:  # the grid holds all channels at once
         assert plan[3] == ctas == -(-nch // plan[2])
     assert plan[4] <= nch
