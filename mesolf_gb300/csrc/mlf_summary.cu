@@ -16,7 +16,7 @@
 // Passes over the movie (HBM-bound streams): a first column pass (t = colsum, and the max), then
 // one pass per iteration but the last that forms s and the next t together (k_si_power), and a
 // last row pass that also computes the image: bg_iter = 5 reads the movie 6 times.  Movies that
-// k_si_power does not take (more than 2048 frames, off the 16-byte grid) need a row and a
+// k_si_power does not take (few frames, more than 2048, off the 16-byte grid) need a row and a
 // column pass per iteration, 2 * bg_iter reads.
 //
 // Column passes: one block per 4 frames x pixel split; each float4 of s is loaded once for
@@ -687,9 +687,9 @@ int summary_block(int64_t T, int w1, int w2, size_t smem_max, size_t* smem) {
 namespace {
 // One power iteration in one pass (k_si_power): CTAs per cluster, frames per CTA and clusters;
 // clusters = 0 where it does not apply (a movie off the 16-byte grid, more than 2048 frames) or the two
-// passes are faster: below 128 frames, but for movies of a few blocks per cluster, whose two launches
-// cost more than the blocks, and from 96 frames for movies far beyond the L2, whose second read comes
-// from HBM.  One pass against two, all of summary_image: 1005 x 1005 px, 16 frames 955 / 608 us, 64
+// passes are faster: below 128 frames, except movies of at most three blocks per cluster, for which two
+// launches cost more than the blocks, and movies of 96 frames and more far beyond the L2, whose second
+// read would come from HBM.  One pass against two, all of summary_image: 1005 x 1005 px, 16 frames 955 / 608 us, 64
 // 1267 / 1161, 96 (388 MB) 1560 / 1587, 128 1731 / 1886; 700 x 700, 32 700 / 504, 96 (188 MB) 969 / 937,
 // 128 1064 / 1090; 465 x 450, 16 495 / 414, 96 623 / 579, 160 707 / 736; 165 x 165 (three blocks), 8 393 /
 // 405, 96 423 / 429.
